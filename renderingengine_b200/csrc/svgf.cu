@@ -13,11 +13,13 @@
 //                at once; the last iteration remodulates (Svgf.cpp:561-577)
 //   k_compose    remodulation when the iteration count is 0
 //
-// Every floating-point expression keeps the reference's operation order and
-// rounding (no contraction: the library is built with --fmad=false and IEEE
-// division / square root), so everything except expf / powf results is
-// bit-identical to the reference's CPU code; history lengths, acceptance and
-// reject reasons are exact.
+// k_temporal keeps the reference's operation order and rounding (no
+// contraction: the library is built with --fmad=false and IEEE division /
+// square root), so the raw, temporal and moment planes, history lengths,
+// acceptance and reject reasons are bit-identical to the reference's CPU
+// code.  The edge weights of k_bootstrap and k_atrous are one exponential
+// each (see edge_exponent), so variance and the filtered planes agree with
+// it to a few float roundings.
 //
 // HBM layout, per pixel of the W x H extent:
 //   history generation (2 x framesInFlight of them): 4 float4 planes
@@ -29,6 +31,8 @@
 //   luminance of the pair)
 //   edge records: float4 (normalised normal, linear depth or -1 where the
 //   surface is not filterable), uint2 (materialId, objectId)
+//   luminance pairs: float2 (temporal, raw signal) for the bootstrap, NaN
+//   where a tap must not count
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -336,11 +340,11 @@ struct Planes {
     uint32_t* hlen;
     float2* moments;
     float* variance;   // bootstrapped temporal variance (ReconstructionFrame::variance)
-    float* var_raw;    // bootstrapped variance of the raw chain
     uint32_t* accepted;
     uint32_t* reject;
     float4* edge;
     uint2* ids;
+    float2* lum;
     float4* chain[2][2][2];  // [svgf=0 / atrous=1][ping][A / B]
 };
 
@@ -436,11 +440,15 @@ __global__ void __launch_bounds__(256) k_temporal(TemporalArgs a) {
     a.pl.edge[i] = make_float4(nn.x, nn.y, nn.z, filterable ? g.depth : -1.0F);
     a.pl.ids[i] = make_uint2(g.mat, g.obj);
     // First inputs of the two chains: the temporal signal (SVGF) and the
-    // current signal (A-Trous only); .w of A = pre-bootstrap variance.
+    // current signal (A-Trous only); .w of A = pre-bootstrap variance.  Both
+    // signals are finite here; their luminance may overflow.
+    const float lum_t = luminance(acc_d, acc_s), lum_r = luminance(safe_d, safe_s);
     a.pl.chain[0][0][0][i] = make_float4(acc_d.x, acc_d.y, acc_d.z, tvar);
-    a.pl.chain[0][0][1][i] = make_float4(acc_s.x, acc_s.y, acc_s.z, luminance(acc_d, acc_s));
+    a.pl.chain[0][0][1][i] = make_float4(acc_s.x, acc_s.y, acc_s.z, lum_t);
     a.pl.chain[1][0][0][i] = make_float4(safe_d.x, safe_d.y, safe_d.z, 0.0F);
-    a.pl.chain[1][0][1][i] = make_float4(safe_s.x, safe_s.y, safe_s.z, luminance(safe_d, safe_s));
+    a.pl.chain[1][0][1][i] = make_float4(safe_s.x, safe_s.y, safe_s.z, lum_r);
+    const float nan = __int_as_float(0x7fffffff);
+    a.pl.lum[i] = make_float2(isfinite(lum_t * lum_t) ? lum_t : nan, isfinite(lum_r * lum_r) ? lum_r : nan);
 }
 
 struct FilterArgs {
@@ -451,57 +459,89 @@ struct FilterArgs {
     const re_gbuffer_pixel* gb;
 };
 
+// log2(1 - z) for z >= 0: -z times a degree-5 Chebyshev fit of
+// -log2(1 - z) / z below 1/8 (relative error 1.5e-8, so the normal weight keeps
+// its precision where it is near 1), the hardware logarithm above, where a
+// power large enough to amplify its 2^-22 has made the weight small; -3e38
+// stands for the logarithm of zero.
+__device__ __forceinline__ float log2_one_minus(float z) {
+    float q = 0x1.5914bep-2F;
+    q = __fmaf_rn(q, z, 0x1.188d4ap-2F);
+    q = __fmaf_rn(q, z, 0x1.7254b8p-2F);
+    q = __fmaf_rn(q, z, 0x1.ec68f2p-2F);
+    q = __fmaf_rn(q, z, 0x1.715480p-1F);
+    q = __fmaf_rn(q, z, 0x1.715476p+0F);
+    float l = -z * q;
+    if (z >= 0.125F) l = fmaxf(__log2f(fmaxf(1.0F - z, 0.0F)), -3.0e38F);
+    return l;
+}
+
+// 2^x, results below 2^-126 flushed to zero.
+__device__ __forceinline__ float exp2_fast(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Base-2 exponent of EdgeWeight's depth and normal terms (Svgf.cpp:246-272):
+// e^(-|dz| / den) * max(0, n . n')^phi = 2^(phi log2(n . n') - |dz| depth_rate)
+// with depth_rate = log2(e) / den, plus `base`.  Both normals are unit, so
+// 1 - n . n' = |n - n'|^2 / 2, which keeps the small angles a rounded dot
+// product loses (phi multiplies its error by 64 to 128).  The luminance term
+// joins the same exponent, so a weight is one ex2 in place of two expf and a
+// powf.
+__device__ __forceinline__ float edge_exponent(float4 c, float4 s, float phi, float depth_rate, float base) {
+    const float dx = c.x - s.x, dy = c.y - s.y, dz = c.z - s.z;
+    const float z = 0.5F * __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+    return __fmaf_rn(phi, log2_one_minus(z), __fmaf_rn(-fabsf(s.w - c.w), depth_rate, base));
+}
+
+constexpr float kLog2E = 1.44269504F;
+
 // BootstrapVariance (Svgf.cpp:584-661) of both chains: the temporal chain
 // with its history lengths and temporal variance, the raw chain with history
-// length 1 and variance 0.
+// length 1 and variance 0.  The bootstrapped variances go into the chains'
+// first inputs, where the first A-Trous iteration reads them.
+//
+// Bound by instruction issue over 49 taps a pixel: a tap reads 32 bytes (edge,
+// IDs, both luminances; NaN marks a luminance that must not count) in place of
+// 88 and takes one exponential in place of expf and powf.  1280x720, radius 3:
+// %BOOT%.
 __global__ void __launch_bounds__(256) k_bootstrap(FilterArgs a) {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= a.W || y >= a.H) return;
+    const int x = int(blockIdx.x * blockDim.x + threadIdx.x);
+    const int y = int(blockIdx.y * blockDim.y + threadIdx.y);
+    const int W = int(a.W), H = int(a.H);
+    if (x >= W || y >= H) return;
     const size_t i = size_t(y) * a.W + x;
     const Cfg& c = a.c;
     const float4 ce = __ldg(a.pl.edge + i);
     float out_t = c.min_variance, out_r = c.min_variance;
     if (ce.w >= 0.0F) {
         const uint2 cid = __ldg(a.pl.ids + i);
-        const V3 cn{ce.x, ce.y, ce.z};
-        const float depth_scale = smax(0.01F, fabsf(ce.w) * 0.02F);
+        const float rate = kLog2E / smax(0.01F, fabsf(ce.w) * 0.02F);
         float w_t = 0.0F, f_t = 0.0F, s_t = 0.0F;
         float w_r = 0.0F, f_r = 0.0F, s_r = 0.0F;
         const int r = int(c.radius);
-        for (int oy = -r; oy <= r; ++oy) {
-            const long long py = (long long)y + oy;
-            if (py < 0 || py >= a.H) continue;
-            for (int ox = -r; ox <= r; ++ox) {
-                const long long px = (long long)x + ox;
-                if (px < 0 || px >= a.W) continue;
-                const size_t j = size_t(py) * a.W + size_t(px);
+        const int x0 = max(x - r, 0), x1 = min(x + r, W - 1);
+        const int y0 = max(y - r, 0), y1 = min(y + r, H - 1);
+        for (int py = y0; py <= y1; ++py) {
+            const size_t row = size_t(py) * a.W;
+#pragma unroll 7
+            for (int px = x0; px <= x1; ++px) {
+                const size_t j = row + px;
                 const float4 se = __ldg(a.pl.edge + j);
-                if (!(se.w >= 0.0F)) continue;
                 const uint2 sid = __ldg(a.pl.ids + j);
-                if (sid.x != cid.x || sid.y != cid.y) continue;
-                const float dw = expf(-fabsf(se.w - ce.w) / depth_scale);
-                const float nw = powf(sclamp(dot(cn, V3{se.x, se.y, se.z}), 0.0F, 1.0F), 32.0F);
-                const float w = dw * nw;
-                if (!isfinite(w) || w <= 0.0F) continue;
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    const float4 sa = __ldg(a.pl.chain[k][0][0] + j);
-                    const float4 sb = __ldg(a.pl.chain[k][0][1] + j);
-                    if (!sig_finite(V3{sa.x, sa.y, sa.z}, V3{sb.x, sb.y, sb.z})) continue;
-                    const float l = sb.w;
-                    const float l2 = l * l;
-                    if (!isfinite(l) || !isfinite(l2)) continue;
-                    if (k == 0) {
-                        f_t += l * w;
-                        s_t += l2 * w;
-                        w_t += w;
-                    } else {
-                        f_r += l * w;
-                        s_r += l2 * w;
-                        w_r += w;
-                    }
-                }
+                if (!(se.w >= 0.0F) || sid.x != cid.x || sid.y != cid.y) continue;
+                const float2 l = __ldg(a.pl.lum + j);
+                const float w = exp2_fast(edge_exponent(ce, se, 32.0F, rate, 0.0F));
+                const float lt = l.x == l.x ? l.x : 0.0F, wt = l.x == l.x ? w : 0.0F;
+                const float lr = l.y == l.y ? l.y : 0.0F, wr = l.y == l.y ? w : 0.0F;
+                f_t = __fmaf_rn(lt, wt, f_t);
+                s_t = __fmaf_rn(lt * lt, wt, s_t);
+                w_t += wt;
+                f_r = __fmaf_rn(lr, wr, f_r);
+                s_r = __fmaf_rn(lr * lr, wr, s_r);
+                w_r += wr;
             }
         }
         const float short_len = float(c.short_history < 1u ? 1u : c.short_history);
@@ -510,7 +550,7 @@ __global__ void __launch_bounds__(256) k_bootstrap(FilterArgs a) {
                                  ? smax(s_t / w_t - (f_t / w_t) * (f_t / w_t), 0.0F)
                                  : 0.0F;
             const float blend = sclamp(float(__ldg(a.pl.hlen + i)) / short_len, 0.0F, 1.0F);
-            const float tv = __ldg(a.pl.chain[0][0][0] + i).w;
+            const float tv = a.pl.chain[0][0][0][i].w;
             const float safe_tv = (isfinite(tv) && tv >= 0.0F) ? tv : sv;
             const float b = lerp1(sv, safe_tv, blend);
             out_t = isfinite(b) ? smax(b, c.min_variance) : c.min_variance;
@@ -525,107 +565,121 @@ __global__ void __launch_bounds__(256) k_bootstrap(FilterArgs a) {
         }
     }
     a.pl.variance[i] = out_t;
-    a.pl.var_raw[i] = out_r;
+    a.pl.chain[0][0][0][i].w = out_t;
+    a.pl.chain[1][0][0][i].w = out_r;
     a.history_variance[4 * i] = out_t;
 }
 
-// One FilterATrous iteration (Svgf.cpp:677-749) for both chains.  FIRST reads
-// the per-pixel variance from the bootstrap planes, later iterations from .w
-// of the chain; LAST remodulates into the frame's atrous / svgf planes.
-template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(256) k_atrous(FilterArgs a, uint32_t step, int ping) {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= a.W || y >= a.H) return;
-    const size_t i = size_t(y) * a.W + x;
+// Two packed float multiply-adds in one instruction (sm_100).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    union U {
+        float2 f;
+        unsigned long long u;
+    };
+    U ua{a}, ub{b}, uc{c}, ud;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(ud.u) : "l"(ua.u), "l"(ub.u), "l"(uc.u));
+    return ud.f;
+}
+
+// Rows of a block of the A-Trous kernel: `step` apart, so the vertical taps of
+// its pixels fall on each other's rows and the block reads R + 4 rows instead
+// of up to 5 R (columns stay consecutive and their loads coalesced).  A step
+// whose bands would not fill the image keeps consecutive rows.
+constexpr uint32_t kAtrousX = 32, kAtrousY = 8;
+__host__ __device__ __forceinline__ uint32_t atrous_row_stride(uint32_t step, uint32_t H) {
+    return step * kAtrousY <= H ? step : 1u;
+}
+
+// One FilterATrous iteration (Svgf.cpp:677-749) for both chains.  The chains'
+// signals are finite and their variances finite and positive (k_temporal and
+// k_bootstrap see to the first inputs, the end of this kernel to the others);
+// only a luminance may overflow, and then the weight is 0 or NaN, and NaN is
+// made 0.  LAST remodulates into the frame's atrous / svgf planes.
+//
+// Bound by instruction issue and L1 (25 taps of 88 bytes).  1280x720, five
+// iterations of a frame: %ATROUS%.
+template <bool LAST>
+__global__ void __launch_bounds__(kAtrousX * kAtrousY) k_atrous(FilterArgs a, int step, int ping) {
+    const int W = int(a.W), H = int(a.H);
+    const uint32_t rs = atrous_row_stride(uint32_t(step), a.H);
+    const int x = int(blockIdx.x * kAtrousX + threadIdx.x);
+    const int y = int((blockIdx.y / rs) * (rs * kAtrousY) + blockIdx.y % rs + threadIdx.y * rs);
+    if (x >= W || y >= H) return;
+    const int i = y * W + x;
     const Cfg& c = a.c;
-    const float* var0[2] = {a.pl.variance, a.pl.var_raw};
     const float4* in_a[2] = {a.pl.chain[0][ping][0], a.pl.chain[1][ping][0]};
     const float4* in_b[2] = {a.pl.chain[0][ping][1], a.pl.chain[1][ping][1]};
 
-    V3 safe_d[2], safe_s[2];
-    float safe_var[2], c_lum[2], lum_den[2];
+    float4 ca[2], cb[2];
+    float rate[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const float4 ca = __ldg(in_a[k] + i);
-        const float4 cb = __ldg(in_b[k] + i);
-        const V3 d{ca.x, ca.y, ca.z}, s{cb.x, cb.y, cb.z};
-        const bool fin = sig_finite(d, s);
-        safe_d[k] = fin ? d : V3{0.0F, 0.0F, 0.0F};
-        safe_s[k] = fin ? s : V3{0.0F, 0.0F, 0.0F};
-        const float v = FIRST ? __ldg(var0[k] + i) : ca.w;
-        safe_var[k] = (isfinite(v) && v >= 0.0F) ? smax(v, c.min_variance) : c.min_variance;
-        c_lum[k] = fin ? cb.w : luminance(safe_d[k], safe_s[k]);
-        lum_den[k] = smax(c.phi_luminance * sqrtf(smax(safe_var[k], 0.0F)), 1.0e-4F);
+        ca[k] = __ldg(in_a[k] + i);
+        cb[k] = __ldg(in_b[k] + i);
+        rate[k] = kLog2E / smax(c.phi_luminance * sqrtf(ca[k].w), 1.0e-4F);
     }
-    V3 out_d[2] = {safe_d[0], safe_d[1]}, out_s[2] = {safe_s[0], safe_s[1]};
-    float out_var[2] = {safe_var[0], safe_var[1]};
+    V3 out_d[2], out_s[2];
+    float out_var[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        out_d[k] = {ca[k].x, ca[k].y, ca[k].z};
+        out_s[k] = {cb[k].x, cb[k].y, cb[k].z};
+        out_var[k] = ca[k].w;
+    }
 
     const float4 ce = __ldg(a.pl.edge + i);
     if (ce.w >= 0.0F) {
         const uint2 cid = __ldg(a.pl.ids + i);
-        const V3 cn{ce.x, ce.y, ce.z};
         const float depth_scale = smax(0.01F, fabsf(ce.w) * 0.01F);
-        const float depth_den = smax(c.phi_depth * depth_scale * float(step), 1.0e-6F);
-        const float kernel[5] = {1.0F, 4.0F, 6.0F, 4.0F, 1.0F};
-        V3 sd[2] = {{0.0F, 0.0F, 0.0F}, {0.0F, 0.0F, 0.0F}};
-        V3 ss[2] = {{0.0F, 0.0F, 0.0F}, {0.0F, 0.0F, 0.0F}};
-        float ws[2] = {0.0F, 0.0F}, wv[2] = {0.0F, 0.0F};
+        const float depth_rate = kLog2E / smax(c.phi_depth * depth_scale * float(step), 1.0e-6F);
+        // log2 of the binomial weights 1 4 6 4 1.
+        const float kernel[5] = {0.0F, 2.0F, 2.5849625F, 2.0F, 0.0F};
+        // Per chain: (d.x, d.y), (d.z, variance), (s.x, s.y), (s.z, unused).
+        float2 acc[2][4];
+        float ws[2] = {0.0F, 0.0F};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) acc[k][h] = make_float2(0.0F, 0.0F);
 #pragma unroll
         for (int ky = -2; ky <= 2; ++ky) {
-            const long long py = (long long)y + (long long)ky * step;
-            if (py < 0 || py >= a.H) continue;
+            const int py = y + ky * step;
+            if (unsigned(py) >= unsigned(H)) continue;
 #pragma unroll
             for (int kx = -2; kx <= 2; ++kx) {
-                const long long px = (long long)x + (long long)kx * step;
-                if (px < 0 || px >= a.W) continue;
-                const size_t j = size_t(py) * a.W + size_t(px);
+                const int px = x + kx * step;
+                if (unsigned(px) >= unsigned(W)) continue;
+                const int j = py * W + px;
                 const float4 se = __ldg(a.pl.edge + j);
-                if (!(se.w >= 0.0F)) continue;  // EdgeWeight == 0
                 const uint2 sid = __ldg(a.pl.ids + j);
-                if (sid.x != cid.x || sid.y != cid.y) continue;
-                // EdgeWeight (Svgf.cpp:246-272): the depth and normal terms
-                // are shared by both chains.
-                const float dw = expf(-fabsf(se.w - ce.w) / depth_den);
-                const float nw = powf(sclamp(dot(cn, V3{se.x, se.y, se.z}), 0.0F, 1.0F), c.phi_normal);
-                const float dn = dw * nw;
-                const float spatial = kernel[kx + 2] * kernel[ky + 2];
+                if (!(se.w >= 0.0F) || sid.x != cid.x || sid.y != cid.y) continue;  // EdgeWeight == 0
+                const float e = edge_exponent(ce, se, c.phi_normal, depth_rate, kernel[kx + 2] + kernel[ky + 2]);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     const float4 sa = __ldg(in_a[k] + j);
                     const float4 sb = __ldg(in_b[k] + j);
-                    const V3 d{sa.x, sa.y, sa.z}, s{sb.x, sb.y, sb.z};
-                    const float sv = FIRST ? __ldg(var0[k] + j) : sa.w;
-                    if (!sig_finite(d, s) || !isfinite(sv) || sv < 0.0F) continue;
-                    const float sl = sb.w;
-                    float ew = 0.0F;
-                    if (isfinite(c_lum[k]) && isfinite(sl)) {
-                        const float lw = expf(-fabsf(sl - c_lum[k]) / lum_den[k]);
-                        ew = dn * lw;
-                        if (!isfinite(ew)) ew = 0.0F;
-                    }
-                    const float w = spatial * ew;
-                    if (!isfinite(w) || w <= 0.0F) continue;
-                    sd[k] = sd[k] + d * w;
-                    ss[k] = ss[k] + s * w;
-                    wv[k] += sv * w * w;
+                    const float w = fmaxf(exp2_fast(__fmaf_rn(-fabsf(sb.w - cb[k].w), rate[k], e)), 0.0F);
+                    const float2 ww = make_float2(w, w);
+                    acc[k][0] = fma2(make_float2(sa.x, sa.y), ww, acc[k][0]);
+                    acc[k][1] = fma2(make_float2(sa.z, sa.w), make_float2(w, w * w), acc[k][1]);
+                    acc[k][2] = fma2(make_float2(sb.x, sb.y), ww, acc[k][2]);
+                    acc[k][3] = fma2(make_float2(sb.z, sb.w), ww, acc[k][3]);
                     ws[k] += w;
                 }
             }
         }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const bool ok = ws[k] > 0.0F && isfinite(ws[k]) && isfinite(wv[k]) && sig_finite(sd[k], ss[k]);
-            V3 fd = ok ? sd[k] / ws[k] : safe_d[k];
-            V3 fs = ok ? ss[k] / ws[k] : safe_s[k];
-            if (!sig_finite(fd, fs)) {
-                fd = safe_d[k];
-                fs = safe_s[k];
+            const V3 sd{acc[k][0].x, acc[k][0].y, acc[k][1].x}, ss{acc[k][2].x, acc[k][2].y, acc[k][3].x};
+            const float wv = acc[k][1].y;
+            if (!(ws[k] > 0.0F && isfinite(ws[k]) && isfinite(wv) && sig_finite(sd, ss))) continue;
+            const V3 fd = sd / ws[k], fs = ss / ws[k];
+            if (sig_finite(fd, fs)) {
+                out_d[k] = fd;
+                out_s[k] = fs;
             }
-            out_d[k] = fd;
-            out_s[k] = fs;
-            const float fv = ok ? wv[k] / (ws[k] * ws[k]) : safe_var[k];
-            out_var[k] = isfinite(fv) ? smax(fv, c.min_variance) : safe_var[k];
+            const float fv = wv / (ws[k] * ws[k]);
+            if (isfinite(fv)) out_var[k] = smax(fv, c.min_variance);
         }
     }
     if (LAST) {
@@ -828,7 +882,7 @@ re_status carve(re_svgf* s, size_t pixels) {
     std::vector<size_t> hist_off;
     for (size_t g = 0; g < gens * 4; ++g) hist_off.push_back(slot(16 * P));
     const size_t o_raw = slot(24 * P), o_tmp = slot(24 * P), o_atr = slot(24 * P), o_svgf = slot(24 * P);
-    const size_t o_hlen = slot(4 * P), o_mom = slot(8 * P), o_var = slot(4 * P), o_varr = slot(4 * P);
+    const size_t o_hlen = slot(4 * P), o_mom = slot(8 * P), o_var = slot(4 * P), o_lum = slot(8 * P);
     const size_t o_acc = slot(4 * P), o_rej = slot(4 * P), o_edge = slot(16 * P), o_ids = slot(8 * P);
     size_t o_chain[2][2][2];
     for (int k = 0; k < 2; ++k)
@@ -852,7 +906,7 @@ re_status carve(re_svgf* s, size_t pixels) {
     pl.hlen = reinterpret_cast<uint32_t*>(base + o_hlen);
     pl.moments = reinterpret_cast<float2*>(base + o_mom);
     pl.variance = reinterpret_cast<float*>(base + o_var);
-    pl.var_raw = reinterpret_cast<float*>(base + o_varr);
+    pl.lum = reinterpret_cast<float2*>(base + o_lum);
     pl.accepted = reinterpret_cast<uint32_t*>(base + o_acc);
     pl.reject = reinterpret_cast<uint32_t*>(base + o_rej);
     pl.edge = reinterpret_cast<float4*>(base + o_edge);
@@ -1085,11 +1139,10 @@ RE_API re_status re_svgf_process(re_svgf* s, const re_svgf_frame_inputs* in, voi
         int ping = 0;
         for (uint32_t it = 0; it < n; ++it) {
             const uint32_t step = 1u << (it < 15u ? it : 15u);
-            const bool first = it == 0, last = it + 1 == n;
-            if (first && last) k_atrous<true, true><<<grid, block, 0, st>>>(fa, step, ping);
-            else if (first) k_atrous<true, false><<<grid, block, 0, st>>>(fa, step, ping);
-            else if (last) k_atrous<false, true><<<grid, block, 0, st>>>(fa, step, ping);
-            else k_atrous<false, false><<<grid, block, 0, st>>>(fa, step, ping);
+            const uint32_t rs = atrous_row_stride(step, H), band = rs * kAtrousY;
+            const dim3 fblock(kAtrousX, kAtrousY), fgrid((W + kAtrousX - 1) / kAtrousX, (H + band - 1) / band * rs);
+            if (it + 1 == n) k_atrous<true><<<fgrid, fblock, 0, st>>>(fa, int(step), ping);
+            else k_atrous<false><<<fgrid, fblock, 0, st>>>(fa, int(step), ping);
             ping ^= 1;
         }
     }
