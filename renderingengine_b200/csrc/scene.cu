@@ -1,6 +1,7 @@
 // Scene residency (IGpuTraversalBackend::BuildOrUpdateScene) and the
 // trace-batch entry points (RecordTraceClosestBatch / RecordTraceAnyBatch).
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -105,7 +106,6 @@ re_status ensure_wide_layout(re_scene* sc) {
 namespace {
 
 constexpr uint32_t kInvalid = 0xffffffffu;
-constexpr int kWarp = 32;
 
 struct HitWriteView {
     const float4* attrs;  // DeviceAttr as 4 x float4
@@ -196,17 +196,12 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& c, unsigned 
 // work counter until the batch is exhausted.
 template <bool ANY, bool COUNT, int STACK>
 __global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
-    const int lane = threadIdx.x & 31;
     TraceOptions opt;
     opt.ignore_instance = kInvalid;
     opt.ignore_primitive = kInvalid;
     opt.shadow = false;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(args.work, uint32_t(kWarp));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= args.count) break;
-        const uint32_t i = base + lane;
+    for (WarpWork w(args.count); w.more(); w.next(args.work)) {
+        const uint32_t i = w.item();
         TraceCounters c{};
         if (i < args.count) {
             const float4* rp = args.rays + size_t(i) * 4u;
@@ -226,39 +221,40 @@ __global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
     }
 }
 
-struct LaunchShape {
-    int grid = 0;
-    int block = 128;
-};
-
-template <typename K>
-LaunchShape persistent_shape(K kernel, int device) {
-    static std::mutex mu;
-    LaunchShape s;
-    int sms = 0;
+// CTAs of `kernel` (128 threads) that fit on the device at once; a fact of the
+// kernel and the device, looked up once per device.
+template <auto K>
+int resident_ctas(int device) {
+    static std::atomic<int> known[64];
+    if (device >= 0 && device < 64 && known[device].load(std::memory_order_relaxed) != 0)
+        return known[device].load(std::memory_order_relaxed);
+    int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, s.block, 0);
-    if (per_sm <= 0) per_sm = 1;
-    s.grid = sms * per_sm;
-    return s;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, 128, 0);
+    const int n = sms * std::max(per_sm, 1);
+    if (device >= 0 && device < 64 && n > 0) known[device].store(n, std::memory_order_relaxed);
+    return std::max(n, 1);
+}
+
+// A grid of resident CTAs, fewer for a batch that gives each warp one ray
+// before it fills them; the work counter is only read when the warps' first
+// batches do not cover the rays (WarpWork), so only then is it cleared.
+template <auto K>
+cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t stream) {
+    const uint32_t full = uint32_t(resident_ctas<K>(sc->device));
+    const uint32_t grid = std::min(full, (args.count + 3u) / 4u);
+    if (uint64_t(grid) * 128u < args.count) {
+        const cudaError_t e = cudaMemsetAsync(args.work, 0, sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return e;
+    }
+    K<<<grid, 128, 0, stream>>>(args);
+    return cudaGetLastError();
 }
 
 template <bool ANY, bool COUNT>
-cudaError_t launch_batch(re_scene* sc, BatchArgs args, cudaStream_t stream) {
-    const uint32_t depth = sc->flat.max_depth;
-    if (depth <= 64) {
-        auto k = trace_batch_kernel<ANY, COUNT, 64>;
-        const LaunchShape s = persistent_shape(k, sc->device);
-        const int need = int((args.count + 127) / 128);
-        k<<<need < s.grid ? need : s.grid, s.block, 0, stream>>>(args);
-    } else {
-        auto k = trace_batch_kernel<ANY, COUNT, 128>;
-        const LaunchShape s = persistent_shape(k, sc->device);
-        const int need = int((args.count + 127) / 128);
-        k<<<need < s.grid ? need : s.grid, s.block, 0, stream>>>(args);
-    }
-    return cudaGetLastError();
+cudaError_t launch_batch(re_scene* sc, const BatchArgs& args, cudaStream_t stream) {
+    if (sc->flat.max_depth <= 64) return launch_batch_k<trace_batch_kernel<ANY, COUNT, 64>>(sc, args, stream);
+    return launch_batch_k<trace_batch_kernel<ANY, COUNT, 128>>(sc, args, stream);
 }
 
 re_status validate_batch(const re_scene* sc, const re_trace_batch* b) {
@@ -313,9 +309,7 @@ re_status run_trace_chunked(re_scene* sc, const re_trace_batch* b, cudaStream_t 
     }
     for (uint32_t k = 0; k < chunks && st == RE_SUCCESS; ++k) {
         const uint32_t off = k * kTraceChunk, cnt = std::min(kTraceChunk, n - off);
-        if (!ok(cudaStreamWaitEvent(stream, in[k], 0)) ||
-            !ok(cudaMemsetAsync(sc->work_counter.ptr, 0, sizeof(uint32_t), stream)))
-            break;
+        if (!ok(cudaStreamWaitEvent(stream, in[k], 0))) break;
         BatchArgs args;
         args.scene = scene_view(sc);
         args.view.attrs = static_cast<const float4*>(sc->attrs.ptr);
@@ -362,7 +356,6 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
         d_hits = static_cast<re_hit_record*>(sc->stage_hits.ptr);
     }
     RE_CUDA_TRY(sc->work_counter.reserve(sizeof(uint32_t)));
-    RE_CUDA_TRY(cudaMemsetAsync(sc->work_counter.ptr, 0, sizeof(uint32_t), stream));
     BatchArgs args;
     args.scene = scene_view(sc);
     args.view.attrs = static_cast<const float4*>(sc->attrs.ptr);

@@ -52,6 +52,40 @@ struct TraceSceneView {
     uint32_t eight_stack;    // most stack entries an eight-wide traversal holds
 };
 
+// A warp's share of a queue of `count` independent items in a persistent
+// kernel.  The first batch is the warp's own by its number (warps of one CTA
+// spread over the queue, so a short queue reaches every SM), later ones come
+// from the global work counter, which starts at zero.  A batch is 32 items
+// while the queue fills the grid's warps; a shorter queue gives each warp the
+// smallest power of two that still covers it, so the rays of a bounce's tail
+// or of a small frame do not wait for 31 others of their warp: there the
+// kernel's time is the slowest warp's, and idle lanes cost nothing.
+struct WarpWork {
+    uint32_t count, warps, chunk, base;
+    __device__ __forceinline__ explicit WarpWork(uint32_t n, uint32_t min_chunk = 1u) : count(n) {
+        warps = gridDim.x * (blockDim.x >> 5);
+        chunk = 32u;
+        while (chunk > min_chunk && (chunk >> 1) * warps >= n) chunk >>= 1;
+        base = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * chunk;
+    }
+    __device__ __forceinline__ bool more() const { return base < count; }
+    // This lane's item of the batch; count when it has none.
+    __device__ __forceinline__ uint32_t item() const {
+        const uint32_t lane = threadIdx.x & 31u;
+        return lane < chunk && base + lane < count ? base + lane : count;
+    }
+    __device__ __forceinline__ void next(uint32_t* work) {
+        const uint32_t first = warps * chunk;
+        if (first >= count) {  // every item was in a first batch
+            base = count;
+            return;
+        }
+        uint32_t b = 0;
+        if ((threadIdx.x & 31) == 0) b = atomicAdd(work, chunk);
+        base = first + __shfl_sync(0xffffffffu, b, 0);
+    }
+};
+
 struct TraceRay {
     f3 o;
     f3 d;
@@ -230,37 +264,6 @@ __device__ __forceinline__ bool slab_test_c(const SlabRayC& r, float x0, float x
                               r.neg_z ? z1 : z0, r.neg_z ? z0 : z1, limit_c, near_out);
 }
 
-// The slab form of a loop: exact (the reference's arithmetic) or
-// conservative (C).
-template <bool C>
-struct SlabOf {
-    using Ray = SlabRay;
-    static __device__ __forceinline__ Ray make(const TraceRay& r) { return make_slab_ray(r); }
-    static __device__ __forceinline__ float limit(float limit_cmp, const Ray&) { return limit_cmp; }
-    static __device__ __forceinline__ bool planes(const Ray& r, float xn, float xf, float yn, float yf, float zn,
-                                                  float zf, float lim, float& near_out) {
-        return slab_test_planes(r, xn, xf, yn, yf, zn, zf, lim, near_out);
-    }
-    static __device__ __forceinline__ bool box(const Ray& r, float x0, float x1, float y0, float y1, float z0,
-                                               float z1, float lim, float& near_out) {
-        return slab_test(r, x0, x1, y0, y1, z0, z1, lim, near_out);
-    }
-};
-template <>
-struct SlabOf<true> {
-    using Ray = SlabRayC;
-    static __device__ __forceinline__ Ray make(const TraceRay& r) { return make_slab_ray_c(r); }
-    static __device__ __forceinline__ float limit(float limit_cmp, const Ray&) { return widen_limit(limit_cmp); }
-    static __device__ __forceinline__ bool planes(const Ray& r, float xn, float xf, float yn, float yf, float zn,
-                                                  float zf, float lim, float& near_out) {
-        return slab_test_planes_c(r, xn, xf, yn, yf, zn, zf, lim, near_out);
-    }
-    static __device__ __forceinline__ bool box(const Ray& r, float x0, float x1, float y0, float y1, float z0,
-                                               float z1, float lim, float& near_out) {
-        return slab_test_c(r, x0, x1, y0, y1, z0, z1, lim, near_out);
-    }
-};
-
 // The six plane vectors of a four-wide node (WideNode: lo / hi per axis for
 // the four children), loaded as entry and exit planes for this ray: the
 // direction signs pick which vector of each axis is loaded as which, so the
@@ -281,6 +284,78 @@ __device__ __forceinline__ WidePlanes load_wide_planes(const float4* w, const R&
     p.zf = __ldg(w + (5 - sz));
     return p;
 }
+
+// (plane - o) * inv of two children at once: packed single-precision adds and
+// multiplies (sm_100), each lane rounded as __fsub_rn / __fmul_rn (a - b is
+// a + (-b)).
+__device__ __forceinline__ float2 plane_pair(float a, float b, float o, float inv) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q;\n\t"
+        "mov.b64 p, {%2, %3};\n\t"
+        "mov.b64 q, {%4, %4};\n\t"
+        "add.rn.f32x2 p, p, q;\n\t"
+        "mov.b64 q, {%5, %5};\n\t"
+        "mul.rn.f32x2 p, p, q;\n\t"
+        "mov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a), "f"(b), "f"(-o), "f"(inv));
+    return r;
+}
+
+// slab_test_planes of the four children of a wide node: entered children get
+// their near distance, the others +inf.
+__device__ __forceinline__ void slab_test_planes4(const SlabRay& r, const WidePlanes& p, float limit_cmp,
+                                                  float (&n)[4]) {
+    const float2 nx0 = plane_pair(p.xn.x, p.xn.y, r.o.x, r.inv.x), nx1 = plane_pair(p.xn.z, p.xn.w, r.o.x, r.inv.x);
+    const float2 fx0 = plane_pair(p.xf.x, p.xf.y, r.o.x, r.inv.x), fx1 = plane_pair(p.xf.z, p.xf.w, r.o.x, r.inv.x);
+    const float2 ny0 = plane_pair(p.yn.x, p.yn.y, r.o.y, r.inv.y), ny1 = plane_pair(p.yn.z, p.yn.w, r.o.y, r.inv.y);
+    const float2 fy0 = plane_pair(p.yf.x, p.yf.y, r.o.y, r.inv.y), fy1 = plane_pair(p.yf.z, p.yf.w, r.o.y, r.inv.y);
+    const float2 nz0 = plane_pair(p.zn.x, p.zn.y, r.o.z, r.inv.z), nz1 = plane_pair(p.zn.z, p.zn.w, r.o.z, r.inv.z);
+    const float2 fz0 = plane_pair(p.zf.x, p.zf.y, r.o.z, r.inv.z), fz1 = plane_pair(p.zf.z, p.zf.w, r.o.z, r.inv.z);
+    auto child = [&](float nx, float ny, float nz, float fx, float fy, float fz) {
+        float tn, tf;
+        asm("max.f32 %0, %1, %2, %3;" : "=f"(tn) : "f"(nx), "f"(ny), "f"(nz));
+        asm("min.f32 %0, %1, %2, %3;" : "=f"(tf) : "f"(fx), "f"(fy), "f"(fz));
+        return !(tf < tn) && tf > r.tmin && tn < limit_cmp ? fmaxf(tn, r.tmin) : INFINITY;
+    };
+    n[0] = child(nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x);
+    n[1] = child(nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y);
+    n[2] = child(nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x);
+    n[3] = child(nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y);
+}
+
+// The slab form of a loop: exact (the reference's arithmetic) or
+// conservative (C).
+template <bool C>
+struct SlabOf {
+    using Ray = SlabRay;
+    static __device__ __forceinline__ Ray make(const TraceRay& r) { return make_slab_ray(r); }
+    static __device__ __forceinline__ float limit(float limit_cmp, const Ray&) { return limit_cmp; }
+    static __device__ __forceinline__ void planes4(const Ray& r, const WidePlanes& p, float lim, float (&n)[4]) {
+        slab_test_planes4(r, p, lim, n);
+    }
+    static __device__ __forceinline__ bool box(const Ray& r, float x0, float x1, float y0, float y1, float z0,
+                                               float z1, float lim, float& near_out) {
+        return slab_test(r, x0, x1, y0, y1, z0, z1, lim, near_out);
+    }
+};
+template <>
+struct SlabOf<true> {
+    using Ray = SlabRayC;
+    static __device__ __forceinline__ Ray make(const TraceRay& r) { return make_slab_ray_c(r); }
+    static __device__ __forceinline__ float limit(float limit_cmp, const Ray&) { return widen_limit(limit_cmp); }
+    static __device__ __forceinline__ void planes4(const Ray& r, const WidePlanes& p, float lim, float (&n)[4]) {
+        float t;
+        n[0] = slab_test_planes_c(r, p.xn.x, p.xf.x, p.yn.x, p.yf.x, p.zn.x, p.zf.x, lim, t) ? t : INFINITY;
+        n[1] = slab_test_planes_c(r, p.xn.y, p.xf.y, p.yn.y, p.yf.y, p.zn.y, p.zf.y, lim, t) ? t : INFINITY;
+        n[2] = slab_test_planes_c(r, p.xn.z, p.xf.z, p.yn.z, p.yf.z, p.zn.z, p.zf.z, lim, t) ? t : INFINITY;
+        n[3] = slab_test_planes_c(r, p.xn.w, p.xf.w, p.yn.w, p.yf.w, p.zn.w, p.zf.w, lim, t) ? t : INFINITY;
+    }
+    static __device__ __forceinline__ bool box(const Ray& r, float x0, float x1, float y0, float y1, float z0,
+                                               float z1, float lim, float& near_out) {
+        return slab_test_c(r, x0, x1, y0, y1, z0, z1, lim, near_out);
+    }
+};
 
 // The next float above a finite x (for either zero the smallest positive
 // subnormal): `y <= x` is `y < next_up(x)` for every finite y, so a
@@ -734,39 +809,20 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
             const float4* w = s.wide + size_t(cur) * 8u;
             const WidePlanes pl = load_wide_planes(w, sr);
             const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
-            if (COUNT) cnt->node_bytes += uint32_t(sizeof(WideNode));
-            float n0 = INFINITY, n1 = INFINITY, n2 = INFINITY, n3 = INFINITY;
+            if (COUNT) {
+                cnt->node_bytes += uint32_t(sizeof(WideNode));
+                cnt->node_tests += uint32_t(ent.x != kWideEmpty) + uint32_t(ent.y != kWideEmpty) +
+                                   uint32_t(ent.z != kWideEmpty) + uint32_t(ent.w != kWideEmpty);
+            }
             // A child's entry matters only when it is entered (finite near):
-            // the others sort last and are neither visited nor pushed.
-            const uint32_t e0 = ent.x, e1 = ent.y, e2 = ent.z, e3 = ent.w;
-            float nn;
-            if (!COUNT || ent.x != kWideEmpty) {  // an empty slot's +inf box is never entered
-                if (COUNT) cnt->node_tests += 1u;
-                if (S::planes(sr, pl.xn.x, pl.xf.x, pl.yn.x, pl.yf.x, pl.zn.x, pl.zf.x, lim, nn)) {
-                    n0 = nn;
-                }
-            }
-            if (!COUNT || ent.y != kWideEmpty) {  // an empty slot's +inf box is never entered
-                if (COUNT) cnt->node_tests += 1u;
-                if (S::planes(sr, pl.xn.y, pl.xf.y, pl.yn.y, pl.yf.y, pl.zn.y, pl.zf.y, lim, nn)) {
-                    n1 = nn;
-                }
-            }
-            if (!COUNT || ent.z != kWideEmpty) {  // an empty slot's +inf box is never entered
-                if (COUNT) cnt->node_tests += 1u;
-                if (S::planes(sr, pl.xn.z, pl.xf.z, pl.yn.z, pl.yf.z, pl.zn.z, pl.zf.z, lim, nn)) {
-                    n2 = nn;
-                }
-            }
-            if (!COUNT || ent.w != kWideEmpty) {  // an empty slot's +inf box is never entered
-                if (COUNT) cnt->node_tests += 1u;
-                if (S::planes(sr, pl.xn.w, pl.xf.w, pl.yn.w, pl.yf.w, pl.zn.w, pl.zf.w, lim, nn)) {
-                    n3 = nn;
-                }
-            }
+            // the others sort last and are neither visited nor pushed.  An
+            // empty slot's +inf box is never entered.
+            float n[4];
+            S::planes4(sr, pl, lim, n);
             // Entered children have finite near distances (near < tMax);
             // the others sort last at +inf.
-            const int down = wide_descend<STACK>(n0, e0, n1, e1, n2, e2, n3, e3, stack, sp, cur, cur_count);
+            const int down =
+                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;
@@ -1119,25 +1175,11 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
             const float4* w = s.wide + size_t(cur) * 8u;
             const WidePlanes pl = load_wide_planes(w, sr);
             const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
-            float n0 = INFINITY, n1 = INFINITY, n2 = INFINITY, n3 = INFINITY;
-            // A child's entry matters only when it is entered (finite near):
-            // the others sort last and are neither visited nor pushed.
-            const uint32_t e0 = ent.x, e1 = ent.y, e2 = ent.z, e3 = ent.w;
-            float nn;
-            // An empty slot's +inf box is never entered.
-            if (S::planes(sr, pl.xn.x, pl.xf.x, pl.yn.x, pl.yf.x, pl.zn.x, pl.zf.x, lim, nn)) {
-                n0 = nn;
-            }
-            if (S::planes(sr, pl.xn.y, pl.xf.y, pl.yn.y, pl.yf.y, pl.zn.y, pl.zf.y, lim, nn)) {
-                n1 = nn;
-            }
-            if (S::planes(sr, pl.xn.z, pl.xf.z, pl.yn.z, pl.yf.z, pl.zn.z, pl.zf.z, lim, nn)) {
-                n2 = nn;
-            }
-            if (S::planes(sr, pl.xn.w, pl.xf.w, pl.yn.w, pl.yf.w, pl.zn.w, pl.zf.w, lim, nn)) {
-                n3 = nn;
-            }
-            const int down = wide_descend<STACK>(n0, e0, n1, e1, n2, e2, n3, e3, stack, sp, cur, cur_count);
+            // As in trace_wide.
+            float n[4];
+            S::planes4(sr, pl, lim, n);
+            const int down =
+                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;
@@ -1389,27 +1431,10 @@ struct WideTraverser {
             const float4* w = s.wide + size_t(cur) * 8u;
             const WidePlanes pl = load_wide_planes(w, sr);
             const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
-            float n0 = INFINITY, n1 = INFINITY, n2 = INFINITY, n3 = INFINITY;
-            uint32_t e0 = 0u, e1 = 0u, e2 = 0u, e3 = 0u;
-            float nn;
-            // An empty slot's +inf box is never entered.
-            if (slab_test_planes(sr, pl.xn.x, pl.xf.x, pl.yn.x, pl.yf.x, pl.zn.x, pl.zf.x, limit_cmp, nn)) {
-                n0 = nn;
-                e0 = ent.x;
-            }
-            if (slab_test_planes(sr, pl.xn.y, pl.xf.y, pl.yn.y, pl.yf.y, pl.zn.y, pl.zf.y, limit_cmp, nn)) {
-                n1 = nn;
-                e1 = ent.y;
-            }
-            if (slab_test_planes(sr, pl.xn.z, pl.xf.z, pl.yn.z, pl.yf.z, pl.zn.z, pl.zf.z, limit_cmp, nn)) {
-                n2 = nn;
-                e2 = ent.z;
-            }
-            if (slab_test_planes(sr, pl.xn.w, pl.xf.w, pl.yn.w, pl.yf.w, pl.zn.w, pl.zf.w, limit_cmp, nn)) {
-                n3 = nn;
-                e3 = ent.w;
-            }
-            const int down = wide_descend<STACK>(n0, e0, n1, e1, n2, e2, n3, e3, stack, sp, cur, cur_count);
+            float n[4];
+            slab_test_planes4(sr, pl, limit_cmp, n);
+            const int down =
+                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;

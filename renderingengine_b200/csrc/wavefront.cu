@@ -178,9 +178,8 @@ template <int STACK, int MODE, int BLOCK = 128>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_intersect(WfDevice d, uint32_t bounce) {
     const uint32_t q = bounce & 1u;
     const uint32_t count = *slot(d, bounce, kSlotRays);
-    uint32_t base;
-    while (fetch(slot(d, bounce, kSlotWorkIntersect), count, base)) {
-        const uint32_t i = base + (threadIdx.x & 31);
+    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkIntersect))) {
+        const uint32_t i = w.item();
         if (i < count)
             d.hit[i] = intersect_one<STACK, MODE>(d.scenes[d.ray_path[q][i] >> kPathBits], d.ray_o[q][i],
                                                   d.ray_d[q][i]);
@@ -1431,9 +1430,8 @@ template <int STACK, bool COUNT, int MODE = 0, int BLOCK = 128>
 __global__ void __launch_bounds__(BLOCK, COUNT ? 1 : 1024 / BLOCK) k_shadow(WfDevice d, uint32_t bounce,
                                                                             unsigned long long* cnt) {
     const uint32_t count = min(*slot(d, bounce, kSlotShadows), d.capacity);
-    uint32_t base;
-    while (fetch(slot(d, bounce, kSlotWorkShadow), count, base)) {
-        const uint32_t i = base + (threadIdx.x & 31);
+    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkShadow))) {
+        const uint32_t i = w.item();
         TraceCounters c{};
         if (i < count) shadow_one<STACK, COUNT, MODE>(d, bounce, i, &c);
         if (COUNT) add_tests(cnt + 3u * kMaxDepth + bounce * 3u, c);
