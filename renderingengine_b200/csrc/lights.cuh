@@ -68,8 +68,21 @@ struct LightContext {
     const float4* env_xf;
 };
 
+// The random numbers of one light sample (dimensions kDimLightSelection ..
+// kDimLightShape3 of `base`), drawn where a light type uses them: an emissive
+// triangle or a sphere takes two shape numbers, an environment four, a point
+// or a directional light none.  Every number is a Philox draw of its own
+// counter, so one that is not drawn changes no other.
 struct LightRandom {
-    float selection, s0, s1, s2, s3;
+    uint32_t pixel, sample, base, stream, seed_lo, seed_hi;
+    __device__ __forceinline__ float draw(uint32_t k) const {
+        return counter_random(pixel, sample, base + k, stream, seed_lo, seed_hi);
+    }
+    __device__ __forceinline__ float selection() const { return draw(kDimLightSelection); }
+    __device__ __forceinline__ float shape0() const { return draw(kDimLightShape0); }
+    __device__ __forceinline__ float shape1() const { return draw(kDimLightShape1); }
+    __device__ __forceinline__ float shape2() const { return draw(kDimLightShape2); }
+    __device__ __forceinline__ float shape3() const { return draw(kDimLightShape3); }
 };
 
 struct LightSample {
@@ -376,34 +389,35 @@ __device__ __forceinline__ float env_pdf(const LightView& v, const float4* xf, f
 // PbrSampleEnvironmentLightL6 (:421-511).
 __device__ __forceinline__ LightSample sample_environment(const LightView& v, const LightContext& c,
                                                           const LightRecord& l, uint32_t idx, float pmf,
-                                                          const LightRandom& u) {
+                                                          float us0, float us1, const LightRandom& u) {
     LightSample s = light_sample_invalid();
     const uint32_t w = v.env_width, h = v.env_height;
     if (!(pmf > 0.f) || w == 0u || h == 0u) return s;
     f3 local;
     float tu, tv, pdf;
     if (v.env_uniform) {
-        const float ct = 1.f - 2.f * u.s0;
+        const float ct = 1.f - 2.f * us0;
         const float st = sqrtf(fmaxf(0.f, 1.f - ct * ct));
-        const float phi = kTwoPi * u.s1;
+        const float phi = kTwoPi * us1;
         local = mk(st * cosf(phi), ct, st * sinf(phi));
         env_uv(local, tu, tv);
         pdf = 1.f / (4.f * kPi);
     } else {
         uint32_t row, col;
         float rp, cp;
-        if (!sample_alias(v.env_rows, h, u.s0, row, rp) || row >= h || !(rp > 0.f)) return s;
-        if (!sample_alias(v.env_cols + size_t(row) * w, w, u.s1, col, cp) || col >= w || !(cp > 0.f)) return s;
+        if (!sample_alias(v.env_rows, h, us0, row, rp) || row >= h || !(rp > 0.f)) return s;
+        if (!sample_alias(v.env_cols + size_t(row) * w, w, us1, col, cp) || col >= w || !(cp > 0.f)) return s;
+        const float us2 = u.shape2(), us3 = u.shape3();
         const float t0 = kPi * float(row) / float(h);
         const float t1 = kPi * float(row + 1u) / float(h);
         const float c0 = cosf(t0), c1 = cosf(t1);
-        const float ct = c0 + (c1 - c0) * u.s3;  // HLSL lerp
+        const float ct = c0 + (c1 - c0) * us3;  // HLSL lerp
         const float st = sqrtf(fmaxf(0.f, 1.f - ct * ct));
-        const float phi = kTwoPi * (float(col) + u.s2) / float(w);
+        const float phi = kTwoPi * (float(col) + us2) / float(w);
         local = mk(st * cosf(phi), ct, st * sinf(phi));
         const float sa = env_texel_solid_angle(v, row);
         if (!(sa > 0.f)) return s;
-        tu = (float(col) + u.s2) / float(w);
+        tu = (float(col) + us2) / float(w);
         tv = acosf(fminf(fmaxf(ct, -1.f), 1.f)) / kPi;
         pdf = rp * cp / sa;
     }
@@ -427,10 +441,16 @@ __device__ __forceinline__ LightSample sample_one_light_body(const LightView& v,
     if (v.alias_count == 0u) return inv;
     uint32_t item;
     float pmf;
-    if (!sample_alias(v.alias, v.alias_count, u.selection, item, pmf)) return inv;
+    if (!sample_alias(v.alias, v.alias_count, u.selection(), item, pmf)) return inv;
     if (item >= v.light_count || !(pmf > 0.f)) return inv;
     const LightRecord l = load_light(v, item);
     if ((l.identity.y & kLightEnabled) == 0u) return inv;
+    // One copy of the two shape draws for the types that take them.
+    float s0 = 0.f, s1 = 0.f;
+    if (l.identity.x >= kLightSphere) {
+        s0 = u.shape0();
+        s1 = u.shape1();
+    }
     switch (l.identity.x) {
         case kLightPoint:
         case kLightSpot:
@@ -438,11 +458,11 @@ __device__ __forceinline__ LightSample sample_one_light_body(const LightView& v,
         case kLightDirectional:
             return sample_directional(l, item, pmf);
         case kLightSphere:
-            return sample_sphere(c, l, item, pmf, u.s0, u.s1);
+            return sample_sphere(c, l, item, pmf, s0, s1);
         case kLightTriangle:
-            return sample_triangle(v, c, l, item, pmf, u.s0, u.s1);
+            return sample_triangle(v, c, l, item, pmf, s0, s1);
         case kLightEnvironment:
-            return item == v.env_light ? sample_environment(v, c, l, item, pmf, u) : inv;
+            return item == v.env_light ? sample_environment(v, c, l, item, pmf, s0, s1, u) : inv;
         default:
             return inv;
     }

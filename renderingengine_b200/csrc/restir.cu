@@ -126,66 +126,133 @@ __device__ __forceinline__ uint32_t neighbor_index(const RestirParams& rp, uint3
 
 }  // namespace
 
-// Initial RIS over `candidates` streamed light samples
-// (RestirInitialV3.comp.hlsl:9-58), the statistics it counts and the
-// history stamps of this frame; the reservoir before temporal reuse.
-__device__ __forceinline__ Reservoir initial_ris(const WfDevice& d, bool live, const FrameParams& fp,
-                                                 const SceneSlot& sc, uint32_t pix, const PrimarySurface& s) {
+namespace {
+
+// What evaluate_unshadowed computes from the surface and the camera alone,
+// once per pixel instead of once per candidate: the same expressions in the
+// same order, so every candidate's target is evaluate_unshadowed's, bit for
+// bit.
+struct RisSurface {
+    f3 n, v;
+    float nov, lambda_v, alpha, spec_den;
+    f3 da, f0;
+};
+__device__ __forceinline__ RisSurface ris_surface(const PrimarySurface& s, f3 cam_pos) {
+    RisSurface r;
+    r.n = normalize3(xyz(s.sn_metal));
+    r.v = normalize3(cam_pos - xyz(s.pos_depth));
+    r.nov = saturate1(dot(r.n, r.v));
+    r.alpha = s.gn_rough.w * s.gn_rough.w;
+    r.lambda_v = 1.f + ggx_lambda(mk(sqrtf(fmaxf(0.f, 1.f - r.nov * r.nov)), 0.f, r.nov), r.alpha);
+    r.spec_den = fmaxf(4.f * r.nov, 1.0e-6f);
+    r.da = mk(fmaxf(s.dalb.x, 0.f), fmaxf(s.dalb.y, 0.f), fmaxf(s.dalb.z, 0.f));
+    r.f0 = mk(fmaxf(s.salb.x, 0.f), fmaxf(s.salb.y, 0.f), fmaxf(s.salb.z, 0.f));
+    return r;
+}
+__device__ __forceinline__ float ris_target(const RisSurface& r, f3 wi, f3 li) {
+    const f3 l = normalize3(wi);
+    const float nol = saturate1(dot(r.n, l));
+    if (!(nol > 0.f) || !(r.nov > 0.f)) return 0.f;
+    const f3 h = normalize3(l + r.v);
+    const float noh = saturate1(dot(r.n, h));
+    const float voh = saturate1(dot(r.v, h));
+    const f3 f = fresnel_schlick(voh, r.f0);
+    const float d = ggx_d(mk(0.f, 0.f, noh), r.alpha);
+    const float g = 1.f / (r.lambda_v + ggx_lambda(mk(0.f, 0.f, nol), r.alpha));
+    const f3 rad = mk(fmaxf(li.x, 0.f), fmaxf(li.y, 0.f), fmaxf(li.z, 0.f));
+    const f3 diffuse = rad * r.da * (f3s(1.f) - f) * (nol * kInvPi);
+    const f3 specular = rad * f * (d * g / r.spec_den);
+    if (!finite3(diffuse) || !finite3(specular)) return 0.f;
+    return luminance_pos(diffuse + specular);
+}
+
+}  // namespace
+
+// The initial RIS over `candidates` streamed light samples
+// (RestirInitialV3.comp.hlsl:9-58) in two parts.  ris_fold walks the stream
+// and leaves the weight sum, M and the selected candidate's index (16 bytes in
+// place of the 256-byte reservoir, so the kernel that runs it neither holds
+// nor writes one); ris_reservoir makes the reservoir before temporal reuse
+// from them, in the kernel that reuses it.
+struct RisFold {
+    float wsum;
+    uint32_t m, win;  // win: kRsInvalidIndex when no candidate was selected
+};
+
+// The random numbers of candidate c of a pixel's stream.
+__device__ __forceinline__ LightRandom ris_numbers(const FrameParams& fp, uint32_t pix, uint32_t c) {
+    return LightRandom{pix, fp.sample * fp.rs.candidates + c, 0u, fp.stream ^ kStreamTagRestir, fp.seed_lo, fp.seed_hi};
+}
+
+__device__ __forceinline__ RisFold ris_fold(const WfDevice& d, const FrameParams& fp, const SceneSlot& sc,
+                                            uint32_t pix, const PrimarySurface& s) {
     const RestirParams& rp = fp.rs;
     const uint32_t C = rp.candidates;
-    Reservoir r = empty_reservoir();
-    const bool sv = surface_valid(s);
     uint32_t n_valid = 0u;
-    if (live && sv && C != 0u) {
+    float wsum = 0.f;
+    uint32_t m = 0u, win = kRsInvalidIndex;
+    if (surface_valid(s)) {
         // An invalid surface makes every candidate invalid (correction 0),
         // leaving the reservoir empty: the loop only runs on valid surfaces.
         uint32_t rs = restir_hash(pix ^ rp.frame_lo ^ 0xa511e9b3u);
         const LightContext lc{xyz(s.pos_depth), xyz(s.gn_rough), xyz(s.sn_metal), fp.env_xf};
-        const uint32_t stream = fp.stream ^ kStreamTagRestir;
-        // Candidate c of this pixel's initial RIS stream (the same light
-        // sample and evaluation whenever it is asked for).
-        auto candidate = [&](uint32_t c) {
-            const uint32_t sample = fp.sample * C + c;
-            LightRandom lr;
-            lr.selection = counter_random(pix, sample, kDimLightSelection, stream, fp.seed_lo, fp.seed_hi);
-            lr.s0 = counter_random(pix, sample, kDimLightShape0, stream, fp.seed_lo, fp.seed_hi);
-            lr.s1 = counter_random(pix, sample, kDimLightShape1, stream, fp.seed_lo, fp.seed_hi);
-            lr.s2 = counter_random(pix, sample, kDimLightShape2, stream, fp.seed_lo, fp.seed_hi);
-            lr.s3 = counter_random(pix, sample, kDimLightShape3, stream, fp.seed_lo, fp.seed_hi);
-            const LightSample ls = sample_one_light<false>(sc.lights, lc, lr);
-            LightSampleV3 ps = to_persistent(sc.lights, rp, ls, pix * C + c);
-            ps.source = make_uint4(pix, s.identity.x, s.identity.y, s.identity.z);
-            return evaluate_candidate(ps, s, fp.cam_pos, rp.scene_gen, rp.candidate_source, kReuseNone, pix);
-        };
         // update_reservoir's fold over the stream, keeping the index of the
         // selected candidate instead of a copy of its 160 bytes: weight sum
         // and M evolve exactly as there (same additions in the same order,
         // same random number per candidate), and the selected candidate is
         // evaluated once more after the loop.  The loop then carries a few
-        // scalars instead of the reservoir.
-        float wsum = 0.f;
-        uint32_t m = 0u, win = kRsInvalidIndex;
+        // scalars instead of the reservoir, and needs of a candidate only
+        // whether it is valid and its weight: the light sample is inlined so
+        // its unused fields and the numbers its type does not take (two of
+        // five draws for a triangle or a sphere) are never computed, and the
+        // surface's share of the target is computed once.  Bound by
+        // instruction issue.  1280x720: 1,380 us
+        // a frame with every number drawn and the surface's share computed per
+        // candidate, 880 us now.
+        const RisSurface rsurf = ris_surface(s, fp.cam_pos);
+#pragma unroll 1
         for (uint32_t c = 0; c < C; ++c) {
-            const Candidate cand = candidate(c);
-            const bool valid = candidate_valid(cand, rp.scene_gen);
+            const LightSample ls = sample_one_light<true>(sc.lights, lc, ris_numbers(fp, pix, c));
+            // to_persistent's and sample_valid's rules, then candidate_valid's
+            // and candidate_weight's on a valid surface (correction 1).
+            bool valid = (ls.flags & kSampleValid) != 0u && ls.light < sc.lights.light_count;
+            if (valid) {
+                const uint4 lid = __ldg(reinterpret_cast<const uint4*>(sc.lights.lights + size_t(ls.light) * 6u + 4));
+                valid = lid.z != kRsInvalidIndex && rp.light_gen != 0u && finite_nonneg1(ls.combined_pdf) &&
+                        finite_nonneg1(ls.selection_pmf) && finite3(ls.wi) && finite3(ls.li);
+            }
+            const float target = valid ? ris_target(rsurf, ls.wi, ls.li) : 0.f;
+            valid = valid && finite_nonneg1(target) && ls.combined_pdf > 0.f;
+            const float weight = valid ? target / ls.combined_pdf : 0.f;
             if (valid) ++n_valid;
-            if (fold_update(wsum, m, valid, candidate_weight(cand, rp.scene_gen), 1u, restir_random(rs))) win = c;
+            if (fold_update(wsum, m, valid, weight, 1u, restir_random(rs))) win = c;
         }
-        r.weight.x = wsum;
-        r.state.x = m;
-        if (win != kRsInvalidIndex) {
-            const Candidate cand = candidate(win);
-            select_candidate(r, cand, candidate_weight(cand, rp.scene_gen));
-        }
+    }
+    atomicAdd(d.counters + kSlotRestirBase + kRsStatGenerated, C);
+    if (n_valid) atomicAdd(d.counters + kSlotRestirBase + kRsStatValid, n_valid);
+    if (C - n_valid) atomicAdd(d.counters + kSlotRestirBase + kRsStatRejected, C - n_valid);
+    return {wsum, m, win};
+}
+
+__device__ __forceinline__ Reservoir ris_reservoir(const WfDevice& d, bool live, const FrameParams& fp,
+                                                   const SceneSlot& sc, uint32_t pix, const PrimarySurface& s,
+                                                   const RisFold& f) {
+    const RestirParams& rp = fp.rs;
+    Reservoir r = empty_reservoir();
+    r.weight.x = f.wsum;
+    r.state.x = f.m;
+    if (f.win != kRsInvalidIndex) {
+        const LightContext lc{xyz(s.pos_depth), xyz(s.gn_rough), xyz(s.sn_metal), fp.env_xf};
+        const LightSample ls = sample_one_light<false>(sc.lights, lc, ris_numbers(fp, pix, f.win));
+        LightSampleV3 ps = to_persistent(sc.lights, rp, ls, pix * rp.candidates + f.win);
+        ps.source = make_uint4(pix, s.identity.x, s.identity.y, s.identity.z);
+        const Candidate cand =
+            evaluate_candidate(ps, s, fp.cam_pos, rp.scene_gen, rp.candidate_source, kReuseNone, pix);
+        select_candidate(r, cand, candidate_weight(cand, rp.scene_gen));
     }
     clamp_m(r, rp.max_m);
     finalize_reservoir(r);
     rs_count(d, kRsStatMClamped, live && (r.state.z & kRsMClamped) != 0u);
-    if (live) {
-        atomicAdd(d.counters + kSlotRestirBase + kRsStatGenerated, C);
-        if (n_valid) atomicAdd(d.counters + kSlotRestirBase + kRsStatValid, n_valid);
-        if (C - n_valid) atomicAdd(d.counters + kSlotRestirBase + kRsStatRejected, C - n_valid);
-    }
     r.state.y = 0u;
     r.h_surface = make_uint4(s.identity.x, s.identity.y, s.identity.z, 0u);
     r.h_scene = make_uint4(rp.scene_gen, rp.light_gen, rp.camera_gen, rp.resolution_gen);
@@ -194,9 +261,9 @@ __device__ __forceinline__ Reservoir initial_ris(const WfDevice& d, bool live, c
     return r;
 }
 
-// PART 1: the initial RIS of one pixel, left in rs_temporal.  PART 2: the
-// temporal reuse (RestirTemporalV3.comp.hlsl:20-215) of that reservoir,
-// written back in place.
+// PART 1: the candidate fold of one pixel, left in the first 16 bytes of its
+// rs_temporal record.  PART 2: the initial reservoir from it and its temporal
+// reuse (RestirTemporalV3.comp.hlsl:20-215), written over the record.
 template <int PART>
 __device__ __forceinline__ void restir_temporal_one(const WfDevice& d, uint32_t v, uint32_t p) {
     const bool live = v != kNoView && d.views[v].rs.enabled != 0u;
@@ -209,11 +276,17 @@ __device__ __forceinline__ void restir_temporal_one(const WfDevice& d, uint32_t 
     const float4* surf_prev = d.prim[rp.parity ^ 1u];
     const PrimarySurface s = load_surface(surf_cur, pp);
     if constexpr (PART == 1) {
-        const Reservoir r = initial_ris(d, live, fp, sc, pix, s);
-        if (live) store_reservoir(d.rs_temporal, p, r);
+        if (!live) return;
+        const RisFold f = ris_fold(d, fp, sc, pix, s);
+        *reinterpret_cast<uint4*>(d.rs_temporal + p) = make_uint4(__float_as_uint(f.wsum), f.m, f.win, 0u);
         return;
     }
-    Reservoir r = live ? load_reservoir(d.rs_temporal, p) : empty_reservoir();
+    RisFold f{0.f, 0u, kRsInvalidIndex};
+    if (live) {
+        const uint4 w = *reinterpret_cast<const uint4*>(d.rs_temporal + p);
+        f = {__uint_as_float(w.x), w.y, w.z};
+    }
+    Reservoir r = ris_reservoir(d, live, fp, sc, pix, s, f);
 
     // Temporal reuse.
     uint32_t rejection = kRejNone;
@@ -372,7 +445,7 @@ __device__ __forceinline__ void restir_spatial_merge(const WfDevice& d, uint32_t
         // The centre's and neighbour k's candidate against this pixel's
         // surface, with its multiple-importance weight: evaluated in the
         // merge and once more for the selected one after it (the merge keeps
-        // the selected source's index, as initial_ris does).
+        // the selected source's index, as the candidate fold does).
         auto centre_candidate = [&](float& w) {
             Candidate cc =
                 evaluate_candidate(center.sel, s, fp.cam_pos, rp.scene_gen, center.prov.x, center.prov.y, pix);

@@ -600,12 +600,7 @@ __device__ __forceinline__ ShadeOut shade_one_v0(const WfDevice& d, const SceneS
     // Next-event estimation (WfPbrBuildDirectShadow).
     if (fp.estimator != 0u && sc.lights.alias_count != 0u && !(fp.estimator == 3u && bounce == 0u && restir_owned)) {
         LightContext lc{hit.p, hit.ng, hit.ns, fp.env_xf};
-        LightRandom lr;
-        lr.selection = rn[kDimLightSelection];
-        lr.s0 = rn[kDimLightShape0];
-        lr.s1 = rn[kDimLightShape1];
-        lr.s2 = rn[kDimLightShape2];
-        lr.s3 = rn[kDimLightShape3];
+        const LightRandom lr{pix, sample, bounce_dim(bounce, 0u), fp.stream, fp.seed_lo, fp.seed_hi};
         const LightSample ls = sample_one_light<false>(sc.lights, lc, lr);
         if ((ls.flags & kSampleValid) != 0u) {
             const BsdfEval ev = bsdf_evaluate<false>(ctx, params, wo, ls.wi);
@@ -949,12 +944,7 @@ __device__ __forceinline__ bool shade_nee(const WfDevice& d, const SceneSlot& sc
     const uint32_t p = st.p, sample = st.id.y, pix = st.id.x;
     const Hit& hit = st.hit;
     LightContext lc{hit.p, hit.ng, hit.ns, fp.env_xf};
-    LightRandom lr;
-    lr.selection = rnd(fp, pix, sample, bounce_dim(bounce, kDimLightSelection));
-    lr.s0 = rnd(fp, pix, sample, bounce_dim(bounce, kDimLightShape0));
-    lr.s1 = rnd(fp, pix, sample, bounce_dim(bounce, kDimLightShape1));
-    lr.s2 = rnd(fp, pix, sample, bounce_dim(bounce, kDimLightShape2));
-    lr.s3 = rnd(fp, pix, sample, bounce_dim(bounce, kDimLightShape3));
+    const LightRandom lr{pix, sample, bounce_dim(bounce, 0u), fp.stream, fp.seed_lo, fp.seed_hi};
     const LightSample ls = sample_one_light<INL>(sc.lights, lc, lr);
     if ((ls.flags & kSampleValid) == 0u) return false;
     const BsdfEval ev = bsdf_evaluate<INL>(st.ctx, st.params, st.wo, ls.wi);
