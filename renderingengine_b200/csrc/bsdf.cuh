@@ -277,12 +277,11 @@ __device__ __forceinline__ float ggx_vndf_pdf(f3 wo, f3 m, float alpha) {
     return ggx_d(m, alpha) * ggx_g1(wo, alpha) * fabsf(dot(wo, m)) / fabsf(wo.z);
 }
 
-// Heitz visible-normal sampling (BsdfSampleGgxVisibleNormalL6, :646-708).
-__device__ __forceinline__ bool ggx_sample_vndf(f3 wo, float alpha, float u1, float u2, f3& m) {
+// Heitz visible-normal sampling (BsdfSampleGgxVisibleNormalL6, :646-708) from
+// the disk point (dx, dy) = sqrt(u1) (cos, sin)(2 pi u2).
+__device__ __forceinline__ bool ggx_vndf_from_disk(f3 wo, float alpha, float dx, float dy, f3& m) {
     m = f3s(0.f);
-    if (wo.z <= kDirEps || alpha < kMinAlpha || !finite3(wo) || !isfinite(u1) || !isfinite(u2) || u1 < 0.f ||
-        u2 < 0.f || u1 >= 1.f || u2 >= 1.f)
-        return false;
+    if (wo.z <= kDirEps || alpha < kMinAlpha || !finite3(wo)) return false;
     f3 v;
     if (!safe_normalize(mk(alpha * wo.x, alpha * wo.y, wo.z), v)) return false;
     if (v.z < 0.f) v = -v;
@@ -294,10 +293,6 @@ __device__ __forceinline__ bool ggx_sample_vndf(f3 wo, float alpha, float u1, fl
         t1 = mk(1.f, 0.f, 0.f);
     }
     const f3 t2 = cross(v, t1);
-    const float r = sqrtf(u1);
-    const float phi = 2.f * kPi * u2;
-    const float dx = r * cosf(phi);
-    float dy = r * sinf(phi);
     const float blend = 0.5f * (1.f + v.z);
     const float base = sqrtf(fmaxf(0.f, 1.f - dx * dx));
     dy = base + (dy - base) * blend;  // lerp(base, dy, blend)
@@ -305,6 +300,14 @@ __device__ __forceinline__ bool ggx_sample_vndf(f3 wo, float alpha, float u1, fl
     const f3 h = t1 * dx + t2 * dy + v * pz;
     if (!safe_normalize(mk(alpha * h.x, alpha * h.y, h.z), m)) return false;
     return m.z > 0.f && dot(wo, m) > 0.f;
+}
+
+__device__ __forceinline__ bool ggx_sample_vndf(f3 wo, float alpha, float u1, float u2, f3& m) {
+    m = f3s(0.f);
+    if (!isfinite(u1) || !isfinite(u2) || u1 < 0.f || u2 < 0.f || u1 >= 1.f || u2 >= 1.f) return false;
+    const float r = sqrtf(u1);
+    const float phi = 2.f * kPi * u2;
+    return ggx_vndf_from_disk(wo, alpha, r * cosf(phi), r * sinf(phi), m);
 }
 
 __device__ __forceinline__ bool ggx_reflection_terms(f3 wo, f3 wi, float alpha, f3& m, float& d, float& g,
@@ -667,24 +670,172 @@ __device__ __forceinline__ BsdfSample bsdf_sample_body(const BsdfContext& c, con
     return r.valid ? r : bsdf_sample_invalid();
 }
 
+// ---------------------------------------------------------------------------
+// The same evaluation and sampling for a whole warp: every lane calls, `live`
+// says which take part, and the lanes meet again after each step.  The
+// functions above leave by early returns at a dozen places, and inlined into
+// a kernel their remainders are compiled apart per exit: a warp then ran them
+// at 12 of 32 lanes.  Steps and expressions are the ones above, so results are
+// bit-identical; the parameters must have passed validate_params (the Shade
+// stage checks them before it records a vertex).
+// ---------------------------------------------------------------------------
+// EvaluateBsdfL6 of the normalised direction wi in frame f.
+__device__ __forceinline__ BsdfEval evaluate_in_frame_warp(bool live, const BsdfContext& c, const BsdfParams& p,
+                                                           const Frame& f, f3 wi_in) {
+    BsdfEval r = bsdf_eval_invalid();
+    f3 wi = f3s(0.f);
+    bool ok = live && safe_normalize(wi_in, wi);
+    if (ok) {
+        const f3 wil = to_local(wi, f);
+        if (p.model == kModelMetallicRoughness) r = eval_metallic_roughness(p, f.wo_local, wil);
+        else if (p.model == kModelLambert) r = eval_lambert(p, f.wo_local, wil);
+        else if (p.model == kModelRoughDielectric) r = eval_rough_dielectric(c, p, f.wo_local, wil);
+        else if (p.model == kModelGgxConductor || p.model == kModelGgxDielectricReflection)
+            r = eval_ggx_reflection(c, p, f.wo_local, wil);
+    }
+    __syncwarp();
+    float corr = 0.f;
+    ok = ok && r.valid && validate_world_event(f.wo, wi, f.ng, r.lobe) && shading_correction(c, f, wi, corr);
+    r.value *= corr;
+    r.diffuse *= corr;
+    r.specular *= corr;
+    r.valid = ok && finite3(r.value) && finite3(r.diffuse) && finite3(r.specular);
+    return r;
+}
+
+__device__ __forceinline__ BsdfEval bsdf_evaluate_warp(bool live, const BsdfContext& c, const BsdfParams& p, f3 wo_in,
+                                                       f3 wi_in) {
+    Frame f;
+    const bool ok = live && build_frame(c, wo_in, f);
+    __syncwarp();
+    return evaluate_in_frame_warp(ok, c, p, f, wi_in);
+}
+
+__device__ __forceinline__ BsdfSample bsdf_sample_warp(bool live, const BsdfContext& c, const BsdfParams& p, f3 wo_in,
+                                                       f3 u) {
+    BsdfSample r = bsdf_sample_invalid();
+    Frame f;
+    bool ok = live && build_frame(c, wo_in, f);
+    __syncwarp();
+    // The disk point every finite model starts from, and which lobe is taken.
+    const float radius = sqrtf(u.y), phi = 2.f * kPi * u.z;
+    const float dx = radius * cosf(phi), dy = radius * sinf(phi);
+    const bool smooth = p.model == kModelSmoothGlass;
+    bool diffuse = false;
+    f3 dir = f3s(0.f);
+    uint32_t lobe = 0u;
+    float eta = 1.f;
+    if (ok) {
+        if (smooth) {
+            r = sample_smooth_glass(c, p, f.wo_local, u.x);
+            ok = r.valid;
+            dir = r.dir;
+            lobe = r.lobe;
+        } else if (p.model == kModelMetallicRoughness) {
+            float pd, ps;
+            ok = metallic_lobe_probabilities(p, f.wo_local, pd, ps);
+            diffuse = u.x < pd;
+            ok = ok && (diffuse || ps > 0.f);
+        } else if (p.model == kModelLambert) {
+            diffuse = true;
+            ok = has_flags(p.lobes, kLobeDiffuseReflection);
+        } else if (p.model != kModelRoughDielectric) {
+            ok = (p.model == kModelGgxConductor || p.model == kModelGgxDielectricReflection) &&
+                 has_flags(p.lobes, kLobeGlossyReflection);
+        }
+    }
+    __syncwarp();
+    f3 m = f3s(0.f);
+    if (ok && !smooth && !diffuse) ok = ggx_vndf_from_disk(f.wo_local, p.roughness * p.roughness, dx, dy, m);
+    __syncwarp();
+    if (ok && !smooth) {
+        if (diffuse) {
+            dir = mk(dx, dy, sqrtf(fmaxf(0.f, 1.f - u.y)));
+            lobe = kLobeDiffuseReflection;
+        } else {
+            bool reflect = true;
+            float pt = 0.f;
+            if (p.model == kModelRoughDielectric) {
+                float fr = 0.f, pr = 0.f;
+                ok = fresnel_dielectric(dot(f.wo_local, m), c.eta_i, c.eta_t, fr) &&
+                     rough_dielectric_probabilities(p, fr, pr, pt);
+                reflect = u.x < pr;
+            }
+            if (reflect) {
+                dir = -f.wo_local + m * (2.f * dot(f.wo_local, m));
+                ok = ok && !(dir.z <= kDirEps);
+                lobe = kLobeGlossyReflection;
+            } else {
+                eta = c.eta_t / c.eta_i;
+                ok = ok && pt > 0.f && refract_local(f.wo_local, m, eta, dir) && !(dir.z >= -kDirEps);
+                lobe = kLobeGlossyTransmission;
+            }
+        }
+    }
+    __syncwarp();
+    f3 wi = f3s(0.f);
+    ok = ok && safe_normalize(to_world(dir, f), wi) && validate_world_event(f.wo, wi, f.ng, lobe);
+    __syncwarp();
+    // EvaluateBsdfL6 builds the frame again around the normalised wo: its axes
+    // are the same, its wo is normalised once more.  (Should that rounding
+    // carry wo across the surface, its own frame is built.)
+    Frame g = f;
+    bool eval = ok && !smooth;
+    if (eval) eval = safe_normalize(f.wo, g.wo);
+    if (eval) {
+        const float side = dot(g.wo, g.ng);
+        if (side < 0.f) {
+            eval = build_frame(c, f.wo, g);
+        } else {
+            g.wo_local = mk(dot(g.wo, g.t), dot(g.wo, g.b), dot(g.wo, g.ns));
+            eval = !(side <= kDirEps || dot(g.wo, g.ns) <= kDirEps) && finite3(g.wo_local) && g.wo_local.z > kDirEps;
+        }
+    }
+    __syncwarp();
+    const BsdfEval e = evaluate_in_frame_warp(eval, c, p, g, wi);
+    if (smooth) {
+        float corr = 0.f;
+        ok = ok && shading_correction(c, f, wi, corr);
+        r.dir = wi;
+        r.value *= corr;
+        r.diffuse *= corr;
+        r.specular *= corr;
+        r.valid = ok && finite3(r.value) && finite3(r.specular);
+    } else {
+        r.dir = wi;
+        r.pdf = e.pdf;
+        r.value = e.value;
+        r.eta = eta;
+        r.diffuse = e.diffuse;
+        r.specular = e.specular;
+        r.measure = kMeasureSolidAngle;
+        r.lobe = lobe;
+        r.delta = false;
+        r.valid = e.valid;
+    }
+    __syncwarp();
+    return r.valid ? r : bsdf_sample_invalid();
+}
+
 // Call-site variants: out-of-line calls keep the caller's register footprint
-// small; inlined bodies avoid the call ABI.  The wavefront Shade kernel is
-// built both ways and the autotuner picks one.
+// small; the inlined warp forms avoid the call ABI.  The wavefront Shade kernel
+// is built both ways and the autotuner picks one.
 static __device__ __noinline__ BsdfEval bsdf_evaluate_call(const BsdfContext& c, const BsdfParams& p, f3 wo, f3 wi) {
     return bsdf_evaluate_body(c, p, wo, wi);
 }
 static __device__ __noinline__ BsdfSample bsdf_sample_call(const BsdfContext& c, const BsdfParams& p, f3 wo, f3 u) {
     return bsdf_sample_body(c, p, wo, u);
 }
+// INLINE: the warp forms above; otherwise one out-of-line call per live lane.
 template <bool INLINE>
-__device__ __forceinline__ BsdfEval bsdf_evaluate(const BsdfContext& c, const BsdfParams& p, f3 wo, f3 wi) {
-    if constexpr (INLINE) return bsdf_evaluate_body(c, p, wo, wi);
-    else return bsdf_evaluate_call(c, p, wo, wi);
+__device__ __forceinline__ BsdfEval bsdf_evaluate(bool live, const BsdfContext& c, const BsdfParams& p, f3 wo, f3 wi) {
+    if constexpr (INLINE) return bsdf_evaluate_warp(live, c, p, wo, wi);
+    else return live ? bsdf_evaluate_call(c, p, wo, wi) : bsdf_eval_invalid();
 }
 template <bool INLINE>
-__device__ __forceinline__ BsdfSample bsdf_sample(const BsdfContext& c, const BsdfParams& p, f3 wo, f3 u) {
-    if constexpr (INLINE) return bsdf_sample_body(c, p, wo, u);
-    else return bsdf_sample_call(c, p, wo, u);
+__device__ __forceinline__ BsdfSample bsdf_sample(bool live, const BsdfContext& c, const BsdfParams& p, f3 wo, f3 u) {
+    if constexpr (INLINE) return bsdf_sample_warp(live, c, p, wo, u);
+    else return live ? bsdf_sample_call(c, p, wo, u) : bsdf_sample_invalid();
 }
 
 }  // namespace re

@@ -45,11 +45,11 @@ __global__ void __launch_bounds__(128) k_bsdf_probe(const float4* __restrict__ q
     p.lobes = __float_as_uint(v[7].w);
     p.complex_fresnel = __float_as_uint(v[8].w);
     const f3 wo = xyz(v[7]), wi = xyz(v[8]), u = xyz(v[9]);
-    const BsdfEval e = bsdf_evaluate<false>(c, p, wo, wi);
-    const BsdfSample s = bsdf_sample<false>(c, p, wo, u);
+    const BsdfEval e = bsdf_evaluate<false>(true, c, p, wo, wi);
+    const BsdfSample s = bsdf_sample<false>(true, c, p, wo, u);
     float pdf_at = 0.f;
     if (s.valid && !s.delta) {
-        const BsdfEval e2 = bsdf_evaluate<false>(c, p, wo, s.dir);
+        const BsdfEval e2 = bsdf_evaluate<false>(true, c, p, wo, s.dir);
         pdf_at = (e2.valid && e2.measure == kMeasureSolidAngle) ? e2.pdf : 0.f;
     }
     float4* o = out + size_t(i) * 8u;

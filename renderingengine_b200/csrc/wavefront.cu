@@ -116,16 +116,13 @@ __global__ void k_raygen(WfDevice d) {
         }
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         d.beta[i] = make_float4(1.f, 1.f, 1.f, 1.f);
-        d.beta_d[i] = z;
-        d.beta_s[i] = z;
+        // beta_d, beta_s and the previous vertex have no value before bounce 1
+        // and are not read before it.
         d.acc_cam[i] = z;
         d.acc_dd[i] = z;
         d.acc_ds[i] = z;
         d.acc_id[i] = z;
         d.acc_is[i] = z;
-        d.prev_pos_pdf[i] = z;
-        d.prev_ng[i] = z;
-        d.prev_ns[i] = z;
         d.ident[i] = make_uint4(pix, fp.sample, 0u, kPathActive | kPathPrevDelta);
         d.gb_pos[i] = z;
         d.gb_nrm[i] = make_float4(0.f, 0.f, 0.f, __uint_as_float(kInv));
@@ -372,6 +369,12 @@ struct Accum {
     f3 cam, dd, ds, id, is;
 };
 
+// The path's diffuse or specular throughput, which starts at the first bounce's
+// scattering event.
+__device__ __forceinline__ f3 split_beta(const float4* plane, uint32_t p, uint32_t bounce) {
+    return bounce == 0u ? f3s(0.f) : from4(plane[p]);
+}
+
 // WfPbrAccumulateTerminal (PbrWavefrontShading.hlsli:127-187).
 __device__ __forceinline__ bool accumulate_terminal(const WfDevice& d, uint32_t p, uint32_t bounce, f3 beta,
                                                     f3 bd, f3 bs, f3 emitted, float mis) {
@@ -416,24 +419,23 @@ __device__ __forceinline__ bool shade_miss(const WfDevice& d, const SceneSlot& s
         }
     }
     if (!finite3(env) || !isfinite(mis)) return false;
-    return accumulate_terminal(d, p, bounce, from4(d.beta[p]), from4(d.beta_d[p]), from4(d.beta_s[p]), env, mis);
+    return accumulate_terminal(d, p, bounce, from4(d.beta[p]), split_beta(d.beta_d, p, bounce),
+                               split_beta(d.beta_s, p, bounce), env, mis);
 }
 
 __device__ __forceinline__ float rnd(const FrameParams& fp, uint32_t path, uint32_t sample, uint32_t dim) {
     return counter_random(path, sample, dim, fp.stream, fp.seed_lo, fp.seed_hi);
 }
 
-// The per-bounce random numbers of one path vertex, dimensions 0..9 of the
-// bounce's block (light selection and shape, BSDF lobe and direction, Russian
-// roulette), drawn in one loop: the same counter-based values as drawing each
-// where it is used, with one copy of the Philox rounds in the Shade code
-// instead of one per draw (the kernel's instruction footprint is what limits
-// its issue rate).
-constexpr uint32_t kBounceDraws = 10u;
+// The per-bounce BSDF and Russian-roulette random numbers of one path vertex,
+// dimensions 5..9 of the bounce's block, drawn in one loop: the same
+// counter-based values as drawing each where it is used, with one copy of the
+// Philox rounds in variant 0's code instead of one per draw.
+constexpr uint32_t kBounceDraws = 5u;
 __device__ __forceinline__ void draw_bounce(const FrameParams& fp, uint32_t pix, uint32_t sample, uint32_t bounce,
                                             float* out) {
 #pragma unroll 1
-    for (uint32_t k = 0; k < kBounceDraws; ++k) out[k] = rnd(fp, pix, sample, bounce_dim(bounce, k));
+    for (uint32_t k = 0; k < kBounceDraws; ++k) out[k] = rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfLobe + k));
 }
 
 // Single-pass Shade (variant 0): records are held until the end of the
@@ -515,8 +517,8 @@ __device__ __forceinline__ ShadeOut shade_one_v0(const WfDevice& d, const SceneS
     const float4 b4 = d.beta[p];
     f3 beta = from4(b4);
     float eta_scale = b4.w;
-    f3 bd = from4(d.beta_d[p]);
-    f3 bs = from4(d.beta_s[p]);
+    f3 bd = split_beta(d.beta_d, p, bounce);
+    f3 bs = split_beta(d.beta_s, p, bounce);
     // Beer-Lambert inside dielectrics (pbr_material_bsdf.hlsli:78-129).
     if (hit.front == 0u && mat.trans_ior.x > 0.f) {
         bool ok = true;
@@ -603,7 +605,7 @@ __device__ __forceinline__ ShadeOut shade_one_v0(const WfDevice& d, const SceneS
         const LightRandom lr{pix, sample, bounce_dim(bounce, 0u), fp.stream, fp.seed_lo, fp.seed_hi};
         const LightSample ls = sample_one_light<false>(sc.lights, lc, lr);
         if ((ls.flags & kSampleValid) != 0u) {
-            const BsdfEval ev = bsdf_evaluate<false>(ctx, params, wo, ls.wi);
+            const BsdfEval ev = bsdf_evaluate<false>(true, ctx, params, wo, ls.wi);
             bool go = ev.valid;
             if (go && (!isfinite(ev.pdf) || !finite3(ev.value))) {
                 atomicAdd(nonfinite, 1u);
@@ -649,8 +651,8 @@ __device__ __forceinline__ ShadeOut shade_one_v0(const WfDevice& d, const SceneS
 
     // BSDF sampling, Russian roulette, next-bounce candidate.
     if (bounce + 1u < fp.max_depth) {
-        const f3 u = mk(rn[kDimBsdfLobe], rn[kDimBsdfU], rn[kDimBsdfV]);
-        const BsdfSample bsmp = bsdf_sample<false>(ctx, params, wo, u);
+        const f3 u = mk(rn[0], rn[kDimBsdfU - kDimBsdfLobe], rn[kDimBsdfV - kDimBsdfLobe]);
+        const BsdfSample bsmp = bsdf_sample<false>(true, ctx, params, wo, u);
         bool valid = bsmp.valid && isfinite(bsmp.pdf) && bsmp.pdf > 0.f && finite3(bsmp.value) &&
                      finite3(bsmp.dir) && !any_negative(bsmp.value);
         if (bsmp.pdf < 0.f) atomicAdd(negpdf, 1u);
@@ -680,7 +682,7 @@ __device__ __forceinline__ ShadeOut shade_one_v0(const WfDevice& d, const SceneS
                 valid = false;
             } else {
                 const float cont = fminf(fmaxf(mag, fp.rr_min), fp.rr_max);
-                const float rr = rn[kDimRussianRoulette];
+                const float rr = rn[kDimRussianRoulette - kDimBsdfLobe];
                 if (rr >= cont) {
                     valid = false;
                 } else {
@@ -852,8 +854,8 @@ __device__ __forceinline__ bool shade_prepare(const WfDevice& d, const SceneSlot
     const float4 b4 = d.beta[p];
     st.beta = from4(b4);
     st.eta_scale = b4.w;
-    st.bd = from4(d.beta_d[p]);
-    st.bs = from4(d.beta_s[p]);
+    st.bd = split_beta(d.beta_d, p, bounce);
+    st.bs = split_beta(d.beta_s, p, bounce);
     // Beer-Lambert inside dielectrics (pbr_material_bsdf.hlsli:78-129).
     if (hit.front == 0u && mat.trans_ior.x > 0.f && mat.atten.w > 0.f) {
         const f3 col = mk(mat.atten.x, mat.atten.y, mat.atten.z);
@@ -934,41 +936,47 @@ struct ShadowRecord {
 };
 
 // Phase 2: next-event estimation (WfPbrBuildDirectShadow,
-// PbrWavefrontShading.hlsli:207-330).  Returns true when a shadow ray is due.
+// PbrWavefrontShading.hlsli:207-330).  Every lane of the warp calls; `live`
+// lanes hold a vertex.  Returns true when a shadow ray is due.
 template <bool INL>
-__device__ __forceinline__ bool shade_nee(const WfDevice& d, const SceneSlot& sc, const FrameParams& fp, uint32_t bounce,
-                                          const ShadeState& st, ShadowRecord& rec, uint32_t* nonfinite,
-                                          uint32_t* negpdf) {
-    if (fp.estimator == 0u || sc.lights.alias_count == 0u || (fp.estimator == 3u && bounce == 0u && st.restir_owned))
-        return false;
-    const uint32_t p = st.p, sample = st.id.y, pix = st.id.x;
+__device__ __forceinline__ bool shade_nee(const WfDevice& d, const SceneSlot& sc, const FrameParams& fp, bool live,
+                                          uint32_t bounce, const ShadeState& st, ShadowRecord& rec,
+                                          uint32_t* nonfinite, uint32_t* negpdf) {
+    bool ok = live && fp.estimator != 0u && sc.lights.alias_count != 0u &&
+              !(fp.estimator == 3u && bounce == 0u && st.restir_owned);
     const Hit& hit = st.hit;
-    LightContext lc{hit.p, hit.ng, hit.ns, fp.env_xf};
-    const LightRandom lr{pix, sample, bounce_dim(bounce, 0u), fp.stream, fp.seed_lo, fp.seed_hi};
-    const LightSample ls = sample_one_light<INL>(sc.lights, lc, lr);
-    if ((ls.flags & kSampleValid) == 0u) return false;
-    const BsdfEval ev = bsdf_evaluate<INL>(st.ctx, st.params, st.wo, ls.wi);
-    if (!ev.valid) return false;
-    if (!isfinite(ev.pdf) || !finite3(ev.value)) {
-        atomicAdd(nonfinite, 1u);
-        return false;
+    LightSample ls = light_sample_invalid();
+    if (ok) {
+        const LightContext lc{hit.p, hit.ng, hit.ns, fp.env_xf};
+        const LightRandom lr{st.id.x, st.id.y, bounce_dim(bounce, 0u), fp.stream, fp.seed_lo, fp.seed_hi};
+        ls = sample_one_light<INL>(sc.lights, lc, lr);
+        ok = (ls.flags & kSampleValid) != 0u;
     }
-    if (ev.pdf < 0.f) {
+    __syncwarp();
+    const BsdfEval ev = bsdf_evaluate<INL>(ok, st.ctx, st.params, st.wo, ls.wi);
+    ok = ok && ev.valid;
+    if (ok && (!isfinite(ev.pdf) || !finite3(ev.value))) {
+        atomicAdd(nonfinite, 1u);
+        ok = false;
+    }
+    if (ok && ev.pdf < 0.f) {
         atomicAdd(negpdf, 1u);
-        return false;
+        ok = false;
     }
     const bool delta = (ls.flags & kSampleDelta) != 0u;
     const float est = delta ? ls.selection_pmf : ls.combined_pdf;
-    if (!isfinite(est)) {
+    if (ok && !isfinite(est)) {
         atomicAdd(nonfinite, 1u);
-        return false;
+        ok = false;
     }
-    if (!(est > 0.f)) {
+    if (ok && !(est > 0.f)) {
         if (est < 0.f) atomicAdd(negpdf, 1u);
-        return false;
+        ok = false;
     }
     const float cosine = fabsf(dot(hit.ng, ls.wi));
-    if (!(cosine > 0.f)) return false;
+    ok = ok && cosine > 0.f;
+    __syncwarp();
+    if (!ok) return false;
     const float mis = delta ? 1.f : power_heuristic(ls.combined_pdf, ev.pdf);
     const f3 scale = ls.li * (cosine * mis / est);
     const f3 cd = bounce == 0u ? st.beta * ev.diffuse * scale : st.bd * ev.value * scale;
@@ -983,22 +991,28 @@ __device__ __forceinline__ bool shade_nee(const WfDevice& d, const SceneSlot& sc
     rec.d = to4(ls.wi, smax);
     rec.cd = to4(cd, est);
     rec.cs = to4(cs, ls.combined_pdf);
-    rec.id = make_uint4(pack_path(p, fp.scene_slot), bounce, ls.light, ls.primitive);
+    rec.id = make_uint4(pack_path(st.p, fp.scene_slot), bounce, ls.light, ls.primitive);
     return true;
 }
 
 // Phase 3: BSDF sampling, Russian roulette and the NextBounce state update
-// (Shade.hlsl:342-455, NextBounce.hlsl:97-112).  Returns true with the next
-// ray when the path continues; otherwise terminates the path.
+// (Shade.hlsl:342-455, NextBounce.hlsl:97-112).  Every lane of the warp calls;
+// `live` lanes hold a vertex.  Returns true with the next ray when the path
+// continues; otherwise terminates it.
 template <bool INL>
-__device__ __forceinline__ bool shade_next(const WfDevice& d, const FrameParams& fp, uint32_t bounce, ShadeState& st,
-                                           float4& n_o, float4& n_d, uint32_t* nonfinite, uint32_t* negpdf) {
+__device__ __forceinline__ bool shade_next(const WfDevice& d, const FrameParams& fp, bool live, uint32_t bounce,
+                                           ShadeState& st, float4& n_o, float4& n_d, uint32_t* nonfinite,
+                                           uint32_t* negpdf) {
     const uint32_t p = st.p, sample = st.id.y, pix = st.id.x;
-    if (bounce + 1u < fp.max_depth) {
-        const f3 u = mk(rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfLobe)),
-                        rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfU)),
-                        rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfV)));
-        const BsdfSample bsmp = bsdf_sample<INL>(st.ctx, st.params, st.wo, u);
+    const bool draws = live && bounce + 1u < fp.max_depth;
+    f3 u = f3s(0.f);
+    if (draws)
+        u = mk(rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfLobe)), rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfU)),
+               rnd(fp, pix, sample, bounce_dim(bounce, kDimBsdfV)));
+    __syncwarp();
+    const BsdfSample bsmp = bsdf_sample<INL>(draws, st.ctx, st.params, st.wo, u);
+    if (!live) return false;
+    if (draws) {
         bool valid = bsmp.valid && isfinite(bsmp.pdf) && bsmp.pdf > 0.f && finite3(bsmp.value) &&
                      finite3(bsmp.dir) && !any_negative(bsmp.value);
         if (bsmp.pdf < 0.f) atomicAdd(negpdf, 1u);
@@ -1105,7 +1119,8 @@ __global__ void __launch_bounds__(128, shade_min_blocks(VARIANT)) k_shade(WfDevi
             }
         }
         ShadowRecord rec;
-        const bool sh = alive && shade_nee<INL>(d, *scp, *fpp, bounce, st, rec, nonfinite, negpdf);
+        __syncwarp();
+        const bool sh = shade_nee<INL>(d, *scp, *fpp, alive, bounce, st, rec, nonfinite, negpdf);
         const uint32_t ss = warp_append(slot(d, bounce, kSlotShadows), sh);
         if (sh) {
             if (ss < d.capacity) {
@@ -1119,7 +1134,7 @@ __global__ void __launch_bounds__(128, shade_min_blocks(VARIANT)) k_shade(WfDevi
             }
         }
         float4 n_o, n_d;
-        const bool nx = alive && shade_next<INL>(d, *fpp, bounce, st, n_o, n_d, nonfinite, negpdf);
+        const bool nx = shade_next<INL>(d, *fpp, alive, bounce, st, n_o, n_d, nonfinite, negpdf);
         const uint32_t ns = warp_append(slot(d, bounce + 1u, kSlotRays), nx);
         if (nx) {
             if (ns < d.capacity) {
@@ -1141,16 +1156,28 @@ __global__ void __launch_bounds__(128, shade_min_blocks(VARIANT)) k_shade(WfDevi
 // Shade state from the record and the path state with the same functions
 // (material parameters, shading frame, view direction) and samples the
 // BSDF, so the next ray is the one the one-kernel Shade emits.
+//
+// Bound by instruction issue and fetch.  All lanes of a warp go through the BSDF
+// together (bsdf_*_warp: branches take turns, then the lanes meet again), and
+// each kernel is held to 128 registers, four CTAs per SM: k_shade_b of a 1080p
+// heightfield frame takes 302 / 153 / 115 us at bounces 0 / 1 / 2 in place of
+// 463 / 283 / 314, and the whole frame 5,564 us, 5,671 without the register bound
+// and 5,569 at five CTAs.
+
+// Smallest batch of a Shade warp on a short queue (WarpWork): unlike a ray's,
+// a vertex's work is the same instructions for every lane, which smaller batches
+// only issue more often.
+constexpr uint32_t kShadeMinBatch = 8u;
+
 template <bool FUSED, int STACK, bool INL>
-__global__ void __launch_bounds__(128) k_shade_a(WfDevice d, uint32_t bounce) {
+__global__ void __launch_bounds__(128, 4) k_shade_a(WfDevice d, uint32_t bounce) {
     const uint32_t q = bounce & 1u;
     const uint32_t count = *slot(d, bounce, kSlotRays);
     uint32_t* work = slot(d, bounce, FUSED ? kSlotWorkIntersect : kSlotWorkShade);
     uint32_t* nonfinite = slot(d, bounce, kSlotNonFinite);
     uint32_t* negpdf = slot(d, bounce, kSlotNegativePdf);
-    uint32_t base;
-    while (fetch(work, count, base)) {
-        const uint32_t i = base + (threadIdx.x & 31);
+    for (WarpWork w(count, kShadeMinBatch); w.more(); w.next(work)) {
+        const uint32_t i = w.item();
         bool alive = i < count;
         ShadeState st;
         const SceneSlot* scp = d.scenes;
@@ -1171,7 +1198,8 @@ __global__ void __launch_bounds__(128) k_shade_a(WfDevice d, uint32_t bounce) {
             }
         }
         ShadowRecord rec;
-        const bool sh = alive && shade_nee<INL>(d, *scp, *fpp, bounce, st, rec, nonfinite, negpdf);
+        __syncwarp();
+        const bool sh = shade_nee<INL>(d, *scp, *fpp, alive, bounce, st, rec, nonfinite, negpdf);
         const uint32_t ss = warp_append(slot(d, bounce, kSlotShadows), sh);
         if (sh) {
             if (ss < d.capacity) {
@@ -1224,8 +1252,8 @@ __device__ __forceinline__ const FrameParams& resume_state(const WfDevice& d, ui
     const float4 b4 = d.beta[st.p];
     st.beta = from4(b4);
     st.eta_scale = b4.w;
-    st.bd = from4(d.beta_d[st.p]);
-    st.bs = from4(d.beta_s[st.p]);
+    st.bd = split_beta(d.beta_d, st.p, bounce);
+    st.bs = split_beta(d.beta_s, st.p, bounce);
     st.ctx.ng = st.hit.ng;
     st.ctx.ns = st.hit.ns;
     f3 tb;
@@ -1247,9 +1275,8 @@ __device__ __forceinline__ void shade_prep_body(const WfDevice& d, uint32_t boun
     const uint32_t count = *slot(d, bounce, kSlotRays);
     uint32_t* work = slot(d, bounce, FUSED ? kSlotWorkIntersect : kSlotWorkShade);
     uint32_t* nonfinite = slot(d, bounce, kSlotNonFinite);
-    uint32_t base;
-    while (fetch(work, count, base)) {
-        const uint32_t i = base + (threadIdx.x & 31);
+    for (WarpWork w(count, kShadeMinBatch); w.more(); w.next(work)) {
+        const uint32_t i = w.item();
         bool alive = i < count;
         ShadeState st;
         if (alive) {
@@ -1284,17 +1311,15 @@ __device__ __forceinline__ void shade_nee_body(const WfDevice& d, uint32_t bounc
     uint32_t* work = slot(d, bounce, kSlotWorkNee);
     uint32_t* nonfinite = slot(d, bounce, kSlotNonFinite);
     uint32_t* negpdf = slot(d, bounce, kSlotNegativePdf);
-    uint32_t base;
-    while (fetch(work, count, base)) {
-        const uint32_t k = base + (threadIdx.x & 31);
-        bool sh = false;
+    for (WarpWork w(count, kShadeMinBatch); w.more(); w.next(work)) {
+        const uint32_t k = w.item();
         ShadowRecord rec;
-        if (k < count) {
-            ShadeState st;
-            const SceneSlot* scp;
-            const FrameParams& fp = resume_state(d, bounce, k, st, scp);
-            sh = shade_nee<true>(d, *scp, fp, bounce, st, rec, nonfinite, negpdf);
-        }
+        ShadeState st;
+        const SceneSlot* scp = d.scenes;
+        const FrameParams* fpp = d.views;
+        if (k < count) fpp = &resume_state(d, bounce, k, st, scp);
+        __syncwarp();
+        const bool sh = shade_nee<true>(d, *scp, *fpp, k < count, bounce, st, rec, nonfinite, negpdf);
         const uint32_t ss = warp_append(slot(d, bounce, kSlotShadows), sh);
         if (sh) {
             if (ss < d.capacity) {
@@ -1317,19 +1342,17 @@ __device__ __forceinline__ void shade_b_body(const WfDevice& d, uint32_t bounce)
     uint32_t* work = slot(d, bounce, kSlotWorkContinue);
     uint32_t* nonfinite = slot(d, bounce, kSlotNonFinite);
     uint32_t* negpdf = slot(d, bounce, kSlotNegativePdf);
-    uint32_t base;
-    while (fetch(work, count, base)) {
-        const uint32_t k = base + (threadIdx.x & 31);
-        bool nx = false;
+    for (WarpWork w(count, kShadeMinBatch); w.more(); w.next(work)) {
+        const uint32_t k = w.item();
         ShadeState st;
         float4 n_o, n_d;
-        if (k < count) {
-            const SceneSlot* scp;
-            const FrameParams& fp = resume_state(d, bounce, k, st, scp);
-            // shade_next ends a path at its last bounce (the three-kernel
-            // form records those vertices too, for their NEE).
-            nx = shade_next<INL>(d, fp, bounce, st, n_o, n_d, nonfinite, negpdf);
-        }
+        const SceneSlot* scp = d.scenes;
+        const FrameParams* fpp = d.views;
+        if (k < count) fpp = &resume_state(d, bounce, k, st, scp);
+        __syncwarp();
+        // shade_next ends a path at its last bounce (the three-kernel form
+        // records those vertices too, for their NEE).
+        const bool nx = shade_next<INL>(d, *fpp, k < count, bounce, st, n_o, n_d, nonfinite, negpdf);
         const uint32_t ns = warp_append(slot(d, bounce + 1u, kSlotRays), nx);
         if (nx) {
             if (ns < d.capacity) {
@@ -1350,9 +1373,9 @@ template <bool FUSED, int STACK>
 __global__ void __launch_bounds__(128) k_shade_prep(WfDevice d, uint32_t bounce) {
     shade_prep_body<FUSED, STACK>(d, bounce);
 }
-__global__ void __launch_bounds__(128) k_shade_nee(WfDevice d, uint32_t bounce) { shade_nee_body(d, bounce); }
+__global__ void __launch_bounds__(128, 4) k_shade_nee(WfDevice d, uint32_t bounce) { shade_nee_body(d, bounce); }
 template <bool INL>
-__global__ void __launch_bounds__(128) k_shade_b(WfDevice d, uint32_t bounce) { shade_b_body<INL>(d, bounce); }
+__global__ void __launch_bounds__(128, 4) k_shade_b(WfDevice d, uint32_t bounce) { shade_b_body<INL>(d, bounce); }
 template <bool FUSED, int STACK, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_shade_prep_capped(WfDevice d, uint32_t bounce) {
     shade_prep_body<FUSED, STACK>(d, bounce);
