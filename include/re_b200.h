@@ -857,7 +857,7 @@ RE_API re_status re_bsdf_probe(const re_bsdf_query* queries, uint32_t count, re_
 /* renderer rebuilding small dynamic meshes between launches of a frame     */
 /* under a fixed memory budget, where a cudaMalloc would synchronise the    */
 /* device.  Every intermediate array lives in one static device array of    */
-/* about 9.3 MB; the call makes no allocation of any kind.                  */
+/* about 5.3 MB; the call makes no allocation of any kind.                  */
 /*   - At most RE_LBVH_STATIC_MAX_TRIANGLES triangles; larger counts fail   */
 /*     with RE_INVALID_ARGUMENT before anything is launched.                */
 /*   - All calls on one device share the scratch: calls that overlap (on    */

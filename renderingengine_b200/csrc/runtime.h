@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -39,12 +40,21 @@ struct alignas(16) DeviceAttr {
 static_assert(sizeof(DeviceAttr) == 64, "attribute record is 64 bytes");
 
 // Scratch buffer that grows on demand and is reused between calls.
+//
+// A pooled buffer comes from the device's scene pool (scene.cu) in place of
+// cudaMalloc.  It is ready on every stream when reserve returns and idle on
+// every stream before release gives it back, as with cudaMalloc and cudaFree,
+// except that an `ordered` one (a build's scratch and results until the build
+// synchronises) is only used on the legacy default stream meanwhile.
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
-    cudaError_t reserve(size_t n);
-    void release();
+    bool pooled = false;
+    cudaError_t reserve(size_t n, bool ordered = false);
+    void release(bool ordered = false);
+    DeviceBuffer() = default;
+    explicit DeviceBuffer(bool from_pool) : pooled(from_pool) {}
     ~DeviceBuffer() { release(); }
 };
 
@@ -53,14 +63,21 @@ struct DeviceBuffer {
 struct re_scene;
 
 namespace re {
-// GPU LBVH build of a scene (Morton codes, radix sort, Karras hierarchy,
-// refit); fills sc->flat and uploads the device layout.
+// GPU LBVH build of a scene from host records (validated by the caller):
+// uploads them and builds as below.
 re_status build_lbvh_on_device(re_scene* sc, const re_canonical_triangle* tris);
-// The same build from CanonicalTraversalTriangle records already in device
-// memory (validated on the device; traversal IDs must be a permutation of
-// 0 .. triangle_count - 1); the leaf-ordered triangle and attribute records
-// are made on the device.
-re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triangle* d_tris);
+// GPU LBVH build (Morton codes, radix sort, Karras hierarchy) from
+// CanonicalTraversalTriangle records in device memory, with the leaf-ordered
+// triangle and attribute records and the four-wide nodes.  `check` validates
+// them on the device; traversal IDs must then be a permutation of 0 ..
+// triangle_count - 1.
+re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triangle* d_tris, bool check);
+// Four-wide nodes from the scene's child-pair nodes, made on the device in
+// `scratch` (wide_scratch_bytes of the child-pair node count).
+size_t wide_scratch_bytes(uint32_t interior);
+re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth);
+// Fills sc->flat's nodes and leaf order when the tree was built on the device.
+re_status host_flat(const re_scene* sc);
 // Child-pair device nodes of sc->flat.
 re_status upload_scene_nodes(re_scene* sc);
 // Leaf-ordered device triangle and attribute records from host records.
@@ -85,37 +102,48 @@ struct re_scene {
     uint32_t generation = 0;
     uint32_t triangle_count = 0;
     uint32_t build_kind = 0;
-    re::FlatBvh flat;               // host copy of the flattened tree
+    // Flattened tree: depth and leaf count, and the host copy of its nodes and
+    // leaf order (for a tree built on the device, made by host_flat when they
+    // are asked for; guarded by flat_mutex).
+    re::FlatBvh flat;
+    std::mutex flat_mutex;
+    uint32_t flat_node_count = 0;
+    float root_lo[3] = {}, root_hi[3] = {};
+    // The tree is this library's own (its child boxes lie in their parents'),
+    // not the caller's flattened nodes.
+    bool own_tree = true;
     re::DeviceLayout layout_meta;   // node_original / root flag (nodes freed after upload)
     // Resident device buffers.
-    re::DeviceBuffer nodes;         // DeviceNode[]
-    re::DeviceBuffer tris;          // DeviceTriangle[]
-    re::DeviceBuffer attrs;         // DeviceAttr[]
+    re::DeviceBuffer nodes{true};         // DeviceNode[]
+    re::DeviceBuffer tris{true};          // DeviceTriangle[]
+    re::DeviceBuffer attrs{true};         // DeviceAttr[]
+    re::DeviceBuffer leaf_order{true};    // source index per leaf (trees built on the device)
     uint32_t device_node_count = 0;
     double build_ms = 0.0;
     double lbvh_gpu_ms = 0.0;    // device time of the GPU LBVH passes
     double lbvh_total_ms = 0.0;
     // Per-scene staging for host-memory trace batches and the work counter of
     // the persistent traversal kernels.
-    re::DeviceBuffer stage_rays;
-    re::DeviceBuffer stage_hits;
-    re::DeviceBuffer work_counter;
-    re::DeviceBuffer counters;
-    // Four-wide nodes over the same triangles (re::WideNode), built on first
-    // use by a renderer tuned for them.
-    re::DeviceBuffer wide_nodes;
+    re::DeviceBuffer stage_rays{true};
+    re::DeviceBuffer stage_hits{true};
+    re::DeviceBuffer work_counter{true};
+    re::DeviceBuffer counters{true};
+    // Four-wide nodes over the same triangles (re::WideNode): made with the
+    // scene for this library's own trees, else on first use by a renderer
+    // tuned for them.
+    re::DeviceBuffer wide_nodes{true};
     uint32_t wide_node_count = 0;
     uint32_t wide_stack_bound = 0;
     // Eight-wide nodes, plain (re::Wide8Node) and compressed (re::Wide8QNode),
     // built on first use by a renderer tuned for them.
-    re::DeviceBuffer eight_nodes, eight_qnodes;
+    re::DeviceBuffer eight_nodes{true}, eight_qnodes{true};
     uint32_t eight_node_count = 0;
     uint32_t eight_stack_bound = 0;
     // Alpha masks: per leaf-ordered triangle texture coordinates + material
     // (2 x float4, made when any triangle is alpha-masked), and the tables
     // of re_scene_set_alpha_masks with their device AlphaView.
     bool alpha_masked = false;
-    re::DeviceBuffer alpha_tc, alpha_materials, alpha_atlas, alpha_view;
+    re::DeviceBuffer alpha_tc{true}, alpha_materials{true}, alpha_atlas{true}, alpha_view{true};
     // Copy streams of chunked host-memory trace batches (created on first use).
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     ~re_scene() {

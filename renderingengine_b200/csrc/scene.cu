@@ -25,12 +25,71 @@ re_status clear_error() {
     return RE_SUCCESS;
 }
 
-cudaError_t DeviceBuffer::reserve(size_t n) {
+namespace {
+
+// Memory of scenes and of their builds.  A cudaMalloc takes about 350 us here
+// and a cudaFree 300, whatever the size, and a scene holds half a dozen
+// buffers: a 606,208-triangle rebuild from device records spent 4 of its 5 ms
+// in them.  The pool keeps at most this much of what is freed, and gives it
+// back when an allocation of the library fails.
+constexpr uint64_t kScenePoolKeeps = 256ull << 20;
+
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pools[64] = {};
+
+cudaError_t scene_pool(int device, cudaMemPool_t* out) {
+    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (g_pools[device] == nullptr) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t keep = kScenePoolKeeps;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        g_pools[device] = pool;
+    }
+    *out = g_pools[device];
+    return cudaSuccess;
+}
+
+// What the pool holds unused goes back to the device.
+void trim_scene_pool(int device) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (device < 0 || device >= 64 || g_pools[device] == nullptr) return;
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(g_pools[device], 0);
+}
+
+cudaError_t raw_allocate(void** ptr, size_t n, bool pooled, int device) {
+    if (!pooled) return cudaMalloc(ptr, n);
+    cudaMemPool_t pool = nullptr;
+    const cudaError_t e = scene_pool(device, &pool);
+    return e != cudaSuccess ? e : cudaMallocFromPoolAsync(ptr, n, pool, cudaStreamLegacy);
+}
+
+}  // namespace
+
+cudaError_t DeviceBuffer::reserve(size_t n, bool ordered) {
     if (n <= bytes && ptr != nullptr) return cudaSuccess;
-    release();
+    release(ordered);
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    e = cudaMalloc(&ptr, n == 0 ? 16 : n);
+    const size_t want = n == 0 ? 16 : n;
+    e = raw_allocate(&ptr, want, pooled, device);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        trim_scene_pool(device);
+        e = raw_allocate(&ptr, want, pooled, device);
+    }
+    if (e == cudaSuccess && pooled && !ordered) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
         ptr = nullptr;
         bytes = 0;
@@ -40,12 +99,17 @@ cudaError_t DeviceBuffer::reserve(size_t n) {
     return cudaSuccess;
 }
 
-void DeviceBuffer::release() {
+void DeviceBuffer::release(bool ordered) {
     if (ptr != nullptr) {
         int cur = 0;
         cudaGetDevice(&cur);
         if (cur != device) cudaSetDevice(device);
-        cudaFree(ptr);
+        if (!pooled) {
+            cudaFree(ptr);
+        } else {
+            if (!ordered) cudaDeviceSynchronize();
+            cudaFreeAsync(ptr, cudaStreamLegacy);
+        }
         if (cur != device) cudaSetDevice(cur);
     }
     ptr = nullptr;
@@ -58,9 +122,10 @@ TraceSceneView scene_view(const re_scene* sc) {
     v.tris = static_cast<const float4*>(sc->tris.ptr);
     v.node_count = sc->device_node_count;
     v.tri_count = sc->triangle_count;
-    const re_software_node& r = sc->flat.nodes[0];
-    v.root_lo[0] = r.bounds_min.x; v.root_lo[1] = r.bounds_min.y; v.root_lo[2] = r.bounds_min.z;
-    v.root_hi[0] = r.bounds_max.x; v.root_hi[1] = r.bounds_max.y; v.root_hi[2] = r.bounds_max.z;
+    for (int a = 0; a < 3; ++a) {
+        v.root_lo[a] = sc->root_lo[a];
+        v.root_hi[a] = sc->root_hi[a];
+    }
     v.wide = static_cast<const float4*>(sc->wide_nodes.ptr);
     v.wide_count = sc->wide_node_count;
     v.wide_stack = sc->wide_stack_bound;
@@ -74,6 +139,8 @@ TraceSceneView scene_view(const re_scene* sc) {
 
 re_status ensure_eight_layout(re_scene* sc) {
     if (sc->eight_node_count != 0u) return RE_SUCCESS;
+    const re_status fst = host_flat(sc);
+    if (fst != RE_SUCCESS) return fst;
     Wide8Layout w;
     build_wide8_layout(sc->flat, w);
     if (w.nodes.empty()) return set_error(RE_INVALID_ARGUMENT, "scene has no hierarchy");
@@ -91,6 +158,8 @@ re_status ensure_eight_layout(re_scene* sc) {
 
 re_status ensure_wide_layout(re_scene* sc) {
     if (sc->wide_node_count != 0u) return RE_SUCCESS;
+    const re_status fst = host_flat(sc);
+    if (fst != RE_SUCCESS) return fst;
     WideLayout w;
     build_wide_layout(sc->flat, w);
     if (w.nodes.empty()) return set_error(RE_INVALID_ARGUMENT, "scene has no hierarchy");
@@ -192,8 +261,15 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& c, unsigned 
     }
 }
 
-// Persistent traversal: every warp pulls 32 consecutive rays from a global
-// work counter until the batch is exhausted.
+// Persistent traversal of a batch.
+__device__ __forceinline__ TraceRay batch_ray(const BatchArgs& args, uint32_t i, uint4& ident) {
+    const float4* rp = args.rays + size_t(i) * 4u;
+    const float4 ot = __ldg(rp + 0);
+    const float4 dt = __ldg(rp + 1);
+    ident = __ldg(reinterpret_cast<const uint4*>(rp + 2));
+    return TraceRay{mk(ot.x, ot.y, ot.z), mk(dt.x, dt.y, dt.z), ot.w, dt.w};
+}
+
 template <bool ANY, bool COUNT, int STACK>
 __global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
     TraceOptions opt;
@@ -204,11 +280,8 @@ __global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
         const uint32_t i = w.item();
         TraceCounters c{};
         if (i < args.count) {
-            const float4* rp = args.rays + size_t(i) * 4u;
-            const float4 ot = __ldg(rp + 0);
-            const float4 dt = __ldg(rp + 1);
-            const uint4 ident = __ldg(reinterpret_cast<const uint4*>(rp + 2));
-            TraceRay ray{mk(ot.x, ot.y, ot.z), mk(dt.x, dt.y, dt.z), ot.w, dt.w};
+            uint4 ident;
+            const TraceRay ray = batch_ray(args, i, ident);
             const TraceHit h = trace<ANY, COUNT, STACK>(args.scene, ray, opt, &c);
             if (COUNT) {
                 if (h.status == 1u) atomicAdd(args.counters + 3, 1ull);
@@ -252,7 +325,7 @@ cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t str
 }
 
 template <bool ANY, bool COUNT>
-cudaError_t launch_batch(re_scene* sc, const BatchArgs& args, cudaStream_t stream) {
+cudaError_t launch_batch(re_scene* sc, BatchArgs args, cudaStream_t stream) {
     if (sc->flat.max_depth <= 64) return launch_batch_k<trace_batch_kernel<ANY, COUNT, 64>>(sc, args, stream);
     return launch_batch_k<trace_batch_kernel<ANY, COUNT, 128>>(sc, args, stream);
 }
@@ -282,7 +355,7 @@ re_status run_trace_chunked(re_scene* sc, const re_trace_batch* b, cudaStream_t 
     const uint32_t n = b->ray_count;
     RE_CUDA_TRY(sc->stage_rays.reserve(size_t(n) * sizeof(re_ray_record)));
     RE_CUDA_TRY(sc->stage_hits.reserve(size_t(n) * sizeof(re_hit_record)));
-    RE_CUDA_TRY(sc->work_counter.reserve(sizeof(uint32_t)));
+    RE_CUDA_TRY(sc->work_counter.reserve(2 * sizeof(uint32_t)));
     if (sc->copy_in == nullptr) {
         RE_CUDA_TRY(cudaStreamCreateWithFlags(&sc->copy_in, cudaStreamNonBlocking));
         RE_CUDA_TRY(cudaStreamCreateWithFlags(&sc->copy_out, cudaStreamNonBlocking));
@@ -355,7 +428,7 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
         d_rays = static_cast<const re_ray_record*>(sc->stage_rays.ptr);
         d_hits = static_cast<re_hit_record*>(sc->stage_hits.ptr);
     }
-    RE_CUDA_TRY(sc->work_counter.reserve(sizeof(uint32_t)));
+    RE_CUDA_TRY(sc->work_counter.reserve(2 * sizeof(uint32_t)));
     BatchArgs args;
     args.scene = scene_view(sc);
     args.view.attrs = static_cast<const float4*>(sc->attrs.ptr);
@@ -415,7 +488,24 @@ re_status upload_scene_nodes(re_scene* sc) {
     RE_CUDA_TRY(cudaMemcpy(sc->nodes.ptr, layout.nodes.data(), layout.nodes.size() * sizeof(DeviceNode),
                            cudaMemcpyHostToDevice));
     sc->device_node_count = uint32_t(layout.nodes.size());
+    const re_software_node& r = sc->flat.nodes[0];
+    sc->root_lo[0] = r.bounds_min.x; sc->root_lo[1] = r.bounds_min.y; sc->root_lo[2] = r.bounds_min.z;
+    sc->root_hi[0] = r.bounds_max.x; sc->root_hi[1] = r.bounds_max.y; sc->root_hi[2] = r.bounds_max.z;
+    sc->flat_node_count = uint32_t(sc->flat.nodes.size());
     return RE_SUCCESS;
+}
+
+// Four-wide nodes of a tree built on the host.  Without the memory for them
+// the scene stands and traces over its child pairs.
+void make_wide_nodes(re_scene* sc) {
+    if (sc->layout_meta.root_is_leaf != 0u) return;
+    DeviceBuffer scratch{true};
+    if (scratch.reserve(wide_scratch_bytes(sc->device_node_count)) != cudaSuccess ||
+        build_wide_on_device(sc, scratch.ptr, nullptr) != RE_SUCCESS) {
+        cudaGetLastError();
+        sc->wide_nodes.release();
+        sc->wide_node_count = sc->wide_stack_bound = 0u;
+    }
 }
 
 re_status upload_scene_geometry(re_scene* sc, const re_canonical_triangle* src_in_leaf_order_or_null,
@@ -562,6 +652,7 @@ RE_API re_status re_scene_create(const re_scene_desc* desc, re_scene** out_scene
         else st = build_lbvh_on_device(sc, desc->triangles);
     } else if (desc->nodes != nullptr) {
         // Caller-flattened SAH: triangles are already in leaf order.
+        sc->own_tree = false;
         sc->flat.nodes.assign(desc->nodes, desc->nodes + desc->node_count);
         sc->flat.leaf_order.resize(desc->triangle_count);
         uint32_t depth = 0, leaves = 0;
@@ -604,6 +695,7 @@ RE_API re_status re_scene_create(const re_scene_desc* desc, re_scene** out_scene
             st = set_error(RE_INVALID_ARGUMENT, err);
         } else {
             st = upload_scene_geometry(sc, nullptr, desc->triangles, sc->flat.leaf_order);
+            if (st == RE_SUCCESS) make_wide_nodes(sc);
         }
     }
     if (st != RE_SUCCESS) {
@@ -638,7 +730,7 @@ RE_API re_status re_scene_create_from_device(const re_scene_desc* desc, re_scene
     const auto t0 = std::chrono::steady_clock::now();
     re_status st = RE_SUCCESS;
     if (cudaSetDevice(sc->device) != cudaSuccess) st = set_error(RE_CUDA_ERROR, "cudaSetDevice failed");
-    else st = build_lbvh_from_device_records(sc, desc->triangles);
+    else st = build_lbvh_from_device_records(sc, desc->triangles, true);
     if (st != RE_SUCCESS) {
         delete sc;
         return st;
@@ -656,10 +748,11 @@ RE_API re_status re_scene_destroy(re_scene* scene) {
 RE_API re_status re_scene_info_get(const re_scene* sc, re_scene_info* out) {
     if (sc == nullptr || out == nullptr) return set_error(RE_INVALID_ARGUMENT, "null argument");
     out->triangle_count = sc->triangle_count;
-    out->node_count = uint32_t(sc->flat.nodes.size());
+    out->node_count = sc->flat_node_count;
     out->max_depth = sc->flat.max_depth;
     out->leaf_count = sc->flat.leaf_count;
-    out->device_bytes = uint64_t(sc->nodes.bytes) + sc->tris.bytes + sc->attrs.bytes + sc->wide_nodes.bytes;
+    out->device_bytes = uint64_t(sc->nodes.bytes) + sc->tris.bytes + sc->attrs.bytes +
+                        sc->leaf_order.bytes + sc->wide_nodes.bytes;
     out->build_ms = sc->build_ms;
     out->node_bytes = sizeof(DeviceNode);
     out->triangle_bytes = sizeof(DeviceTriangle);
@@ -670,6 +763,8 @@ RE_API re_status re_scene_info_get(const re_scene* sc, re_scene_info* out) {
 RE_API re_status re_scene_export_flat(const re_scene* sc, re_software_node* nodes, uint32_t node_capacity,
                                       uint32_t* leaf_order, uint32_t order_capacity) {
     if (sc == nullptr) return set_error(RE_INVALID_ARGUMENT, "scene is null");
+    const re_status fst = host_flat(sc);
+    if (fst != RE_SUCCESS) return fst;
     if (nodes != nullptr) {
         if (node_capacity < sc->flat.nodes.size()) return set_error(RE_INVALID_ARGUMENT, "node capacity too small");
         std::memcpy(nodes, sc->flat.nodes.data(), sc->flat.nodes.size() * sizeof(re_software_node));

@@ -52,10 +52,11 @@ struct Request {
     size_t result_bytes = 0;
 };
 
-// Device bytes a resident scene takes: BVH nodes, triangles and attributes
-// (re_scene_info.device_bytes) plus the renderer's per-slot tables.
+// Device bytes a resident scene is charged: child-pair nodes, triangles and
+// attributes (re_scene_info.device_bytes without the four-wide nodes, which
+// have never been part of the charge) plus the renderer's per-slot tables.
 uint64_t scene_bytes(const SceneRecord& rec, const re_scene_info& info) {
-    return info.device_bytes + uint64_t(rec.tris.size()) * 4u + rec.materials.size() * sizeof(re_material) +
+    return info.device_bytes - rec.scene->wide_nodes.bytes + uint64_t(rec.tris.size()) * 4u + rec.materials.size() * sizeof(re_material) +
            rec.lights.size() * (sizeof(re_light) + 24u) + rec.fixtures.size() * sizeof(re_float4);
 }
 
