@@ -88,6 +88,9 @@ re_status upload_scene_triangles(re_scene* sc, const re_canonical_triangle* src_
 // Film mean of paths [offset, offset + n) into pinned host memory, queued on
 // `s` without synchronising.
 re_status renderer_copy_mean_async(re_renderer* r, uint32_t offset, uint32_t n, void* host_dst, cudaStream_t s);
+// Adds the sample last rendered into paths [src, src + n) to the film of paths
+// [dst, dst + n), queued on `s`.
+re_status renderer_add_sample_async(re_renderer* r, uint32_t dst, uint32_t src, uint32_t n, cudaStream_t s);
 // Allocates the ReSTIR state now (so a budget can account for it).
 re_status renderer_reserve_restir(re_renderer* r);
 // Device bytes held by the renderer (path pool, tables, ReSTIR state).

@@ -40,6 +40,11 @@ struct SceneRecord {
     uint64_t bytes = 0;
 };
 
+// A step takes further samples of its requests up to this many paths in all:
+// a launch of fewer leaves most of the device idle (a 256x256 Cornell frame
+// takes 320 us, a 1280x720 one with 14 times the paths 1,530).
+constexpr uint32_t kStepPaths = 1u << 20;
+
 struct Request {
     uint64_t id = 0, scene_key = 0;
     re_frame_constants frame{};
@@ -56,8 +61,9 @@ struct Request {
 // attributes (re_scene_info.device_bytes without the four-wide nodes, which
 // have never been part of the charge) plus the renderer's per-slot tables.
 uint64_t scene_bytes(const SceneRecord& rec, const re_scene_info& info) {
-    return info.device_bytes - rec.scene->wide_nodes.bytes + uint64_t(rec.tris.size()) * 4u + rec.materials.size() * sizeof(re_material) +
-           rec.lights.size() * (sizeof(re_light) + 24u) + rec.fixtures.size() * sizeof(re_float4);
+    return info.device_bytes - rec.scene->wide_nodes.bytes + uint64_t(rec.tris.size()) * 4u +
+           rec.materials.size() * sizeof(re_material) + rec.lights.size() * (sizeof(re_light) + 24u) +
+           rec.fixtures.size() * sizeof(re_float4);
 }
 
 // Charge of a scene before it is built: an upper bound of scene_bytes (a
@@ -288,22 +294,57 @@ void admit(re_server* s, double now) {
     }
 }
 
-// One step: one sample of every active request, in the launches of
-// plan_launches (requests grouped by scene, under the path budget).
+// One step: the next sample of every active request, and while the step is
+// small further samples of requests that do not reuse their last frame (not
+// ReSTIR), each in a path range of its own whose sample is added to the
+// request's film after the launches, in order; in the launches of plan_launches
+// (requests grouped by scene, under the path budget).
 re_status step(re_server* s) {
-    const size_t n = s->active.size();
+    struct Extra {
+        uint32_t request, offset;  // index into active; path range of its pixels
+    };
+    const size_t active = s->active.size();
+    struct Extras : std::vector<Extra> {
+        re_server* s;
+        const std::vector<uint64_t> owners;  // the requests, by Extra::request
+        explicit Extras(re_server* server) : s(server), owners(server->active) {}
+        // The next launch may reuse the ranges: it is stream-ordered after these.
+        ~Extras() {
+            for (const Extra& e : *this) s->paths.release(e.offset, s->requests.at(owners[e.request]).pixels);
+        }
+    } extras(s);
+    std::vector<uint32_t> taken(active, 1u);  // samples of each request in this step
+    uint64_t paths = 0;
+    for (uint64_t id : s->active) paths += s->requests.at(id).pixels;
+    for (bool more = true; more;) {
+        more = false;
+        for (size_t k = 0; k < active && active + extras.size() < s->desc.max_batch_views; ++k) {
+            const Request& q = s->requests.at(s->active[k]);
+            uint32_t off = 0;
+            if (q.frame.sampling.w == RE_ESTIMATOR_RESTIR_PRIMARY || q.samples_done + taken[k] >= q.spp ||
+                paths + q.pixels > kStepPaths || !s->paths.allocate(q.pixels, off))
+                continue;
+            extras.push_back({uint32_t(k), off});
+            ++taken[k];
+            paths += q.pixels;
+            more = true;
+        }
+    }
+    const size_t n = active + extras.size();
     std::vector<re_view_desc> views(n);
     std::vector<re_frame_constants> frames(n);
-    std::vector<uint32_t> slots(n), pixels(n);
+    std::vector<uint32_t> slots(n), pixels(n), next(active, 0u);
     for (size_t k = 0; k < n; ++k) {
-        Request& q = s->requests.at(s->active[k]);
+        const bool extra = k >= active;
+        const size_t of = extra ? extras[k - active].request : k;
+        Request& q = s->requests.at(s->active[of]);
         frames[k] = q.frame;
-        frames[k].image.z = q.frame.image.z + q.samples_done;
+        frames[k].image.z = q.frame.image.z + q.samples_done + next[of]++;
         re_view_desc& v = views[k];
         v.frame = &frames[k];
         v.scene_slot = uint32_t(s->scenes.at(q.scene_key).slot);
-        v.path_offset = q.offset;
-        v.accumulate = q.samples_done > 0 ? 1u : 0u;
+        v.path_offset = extra ? extras[k - active].offset : q.offset;
+        v.accumulate = !extra && q.samples_done > 0 ? 1u : 0u;
         v.view_key = q.id;
         slots[k] = v.scene_slot;
         pixels[k] = q.pixels;
@@ -320,10 +361,18 @@ re_status step(re_server* s) {
         if (st != RE_SUCCESS) return st;
         ++s->stats.launches;
     }
+    // A request's extra samples were taken in order, so this adds them in order.
+    for (const Extra& e : extras) {
+        const Request& q = s->requests.at(s->active[e.request]);
+        st = renderer_add_sample_async(s->renderer, q.offset, e.offset, q.pixels, s->stream);
+        if (st != RE_SUCCESS) return st;
+    }
     std::vector<uint64_t> still;
-    for (uint64_t id : s->active) {
+    for (size_t k = 0; k < active; ++k) {
+        const uint64_t id = s->active[k];
         Request& q = s->requests.at(id);
-        if (++q.samples_done < q.spp) {
+        q.samples_done += taken[k];
+        if (q.samples_done < q.spp) {
             still.push_back(id);
             continue;
         }

@@ -3073,6 +3073,22 @@ re_status renderer_copy_mean_async(re_renderer* r, uint32_t offset, uint32_t n, 
     return RE_SUCCESS;
 }
 
+// Resolve's accumulation of a sample rendered into another path range.
+__global__ void k_add_sample(float4* film, const float4* sample, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 p = film[i], s = sample[i];
+    film[i] = make_float4(p.x + s.x, p.y + s.y, p.z + s.z, p.w + 1.f);
+}
+
+re_status renderer_add_sample_async(re_renderer* r, uint32_t dst, uint32_t src, uint32_t n, cudaStream_t s) {
+    if (uint64_t(dst) + n > r->capacity || uint64_t(src) + n > r->capacity)
+        return set_error(RE_INVALID_ARGUMENT, "path range exceeds the capacity");
+    k_add_sample<<<(n + 255) / 256, 256, 0, s>>>(r->dev.film_sum + dst, r->dev.sample_out + src, n);
+    RE_CUDA_TRY(cudaGetLastError());
+    return RE_SUCCESS;
+}
+
 re_status renderer_reserve_restir(re_renderer* r) { return ensure_restir_buffers(r); }
 
 uint64_t renderer_device_bytes(const re_renderer* r) {
