@@ -62,9 +62,10 @@ struct TraceSceneView {
 // kernel's time is the slowest warp's, and idle lanes cost nothing.
 struct WarpWork {
     uint32_t count, warps, chunk, base;
-    __device__ __forceinline__ explicit WarpWork(uint32_t n, uint32_t min_chunk = 1u) : count(n) {
+    __device__ __forceinline__ explicit WarpWork(uint32_t n, uint32_t min_chunk = 1u, uint32_t max_chunk = 32u)
+        : count(n) {
         warps = gridDim.x * (blockDim.x >> 5);
-        chunk = 32u;
+        chunk = max_chunk;
         while (chunk > min_chunk && (chunk >> 1) * warps >= n) chunk >>= 1;
         base = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * chunk;
     }
@@ -179,10 +180,36 @@ __device__ __forceinline__ bool slab_test_planes(const SlabRay& r, float xn, flo
     return hit;
 }
 
+// (plane - o) * inv of two planes at once: packed single-precision adds and
+// multiplies (sm_100), each lane rounded as __fsub_rn / __fmul_rn (a - b is
+// a + (-b)).
+__device__ __forceinline__ float2 plane_pair(float a, float b, float o, float inv) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q;\n\t"
+        "mov.b64 p, {%2, %3};\n\t"
+        "mov.b64 q, {%4, %4};\n\t"
+        "add.rn.f32x2 p, p, q;\n\t"
+        "mov.b64 q, {%5, %5};\n\t"
+        "mul.rn.f32x2 p, p, q;\n\t"
+        "mov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a), "f"(b), "f"(-o), "f"(inv));
+    return r;
+}
+
+// As slab_test_planes, from the lower and upper plane of each axis.
 __device__ __forceinline__ bool slab_test(const SlabRay& r, float x0, float x1, float y0, float y1,
                                           float z0, float z1, float limit_cmp, float& near_out) {
-    return slab_test_planes(r, r.neg_x ? x1 : x0, r.neg_x ? x0 : x1, r.neg_y ? y1 : y0, r.neg_y ? y0 : y1,
-                            r.neg_z ? z1 : z0, r.neg_z ? z0 : z1, limit_cmp, near_out);
+    const float2 x = plane_pair(x0, x1, r.o.x, r.inv.x), y = plane_pair(y0, y1, r.o.y, r.inv.y),
+                 z = plane_pair(z0, z1, r.o.z, r.inv.z);
+    float tn, tf;
+    asm("max.f32 %0, %1, %2, %3;"
+        : "=f"(tn) : "f"(r.neg_x ? x.y : x.x), "f"(r.neg_y ? y.y : y.x), "f"(r.neg_z ? z.y : z.x));
+    asm("min.f32 %0, %1, %2, %3;"
+        : "=f"(tf) : "f"(r.neg_x ? x.x : x.y), "f"(r.neg_y ? y.x : y.y), "f"(r.neg_z ? z.x : z.y));
+    const bool hit = !(tf < tn) && tf > r.tmin && tn < limit_cmp;
+    near_out = fmaxf(tn, r.tmin);
+    return hit;
 }
 
 // Conservative slab test (traversal modes 7 and 8): each plane distance is
@@ -285,23 +312,6 @@ __device__ __forceinline__ WidePlanes load_wide_planes(const float4* w, const R&
     return p;
 }
 
-// (plane - o) * inv of two children at once: packed single-precision adds and
-// multiplies (sm_100), each lane rounded as __fsub_rn / __fmul_rn (a - b is
-// a + (-b)).
-__device__ __forceinline__ float2 plane_pair(float a, float b, float o, float inv) {
-    float2 r;
-    asm("{\n\t.reg .b64 p, q;\n\t"
-        "mov.b64 p, {%2, %3};\n\t"
-        "mov.b64 q, {%4, %4};\n\t"
-        "add.rn.f32x2 p, p, q;\n\t"
-        "mov.b64 q, {%5, %5};\n\t"
-        "mul.rn.f32x2 p, p, q;\n\t"
-        "mov.b64 {%0, %1}, p;\n\t}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a), "f"(b), "f"(-o), "f"(inv));
-    return r;
-}
-
 // slab_test_planes of the four children of a wide node: entered children get
 // their near distance, the others +inf.
 __device__ __forceinline__ void slab_test_planes4(const SlabRay& r, const WidePlanes& p, float limit_cmp,
@@ -366,6 +376,20 @@ __device__ __forceinline__ float next_up(float x) {
     return x >= 0.0f ? __uint_as_float((u & 0x7fffffffu) + 1u) : __uint_as_float(u - 1u);
 }
 
+// What makes a closest hit independent of the order of visits.  A box's near
+// distance and a triangle's t are rounded separately, so a box may start an
+// ulp or two behind the triangle in it; with another hit between the two, the
+// loop that meets the other one first prunes the box and the loop that meets
+// the box first does not.  A loop that must agree with another loop's order
+// therefore visits and tests up to `reach` of its best hit, 2^-16 beyond it
+// (a hundred times any such gap), and notes whether a second triangle was
+// hit within that margin.  If none was, every order of visits over the same leaf
+// boxes ends with this hit; also if the hit triangle's own box starts no later
+// than its t, since then no hit prunes it (and so between the two triangles of
+// a mesh edge).  Otherwise, or when two distances are equal, the hit is
+// `contested`, and the caller takes the other loop's.
+__device__ __forceinline__ float reach(float t) { return next_up(__fmaf_rn(fabsf(t), 0x1p-16f, t)); }
+
 // Moller-Trumbore in the CPU mirror's exact operation order.
 __device__ __forceinline__ bool tri_test(const TraceRay& r, float4 p0, float4 e1v, float4 e2v,
                                          float limit_cmp, float& t_out, float& u_out,
@@ -389,8 +413,8 @@ __device__ __forceinline__ bool tri_test(const TraceRay& r, float4 p0, float4 e1
     const float v = __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(r.d.x, qx), __fmul_rn(r.d.y, qy)), __fmul_rn(r.d.z, qz)), inv);
     if (!(v >= 0.0f && __fadd_rn(u, v) <= 1.0f)) return false;
     const float t = __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(e2x, qx), __fmul_rn(e2y, qy)), __fmul_rn(e2z, qz)), inv);
-    const bool within_limit = t < limit_cmp;
-    if (!(isfinite(t) && t > r.tmin && t < r.tmax && within_limit)) return false;
+    // limit_cmp is at most tMax, so the reference's finite and tMax tests follow.
+    if (!(t > r.tmin && t < limit_cmp)) return false;
     t_out = t;
     u_out = u;
     v_out = v;
@@ -738,7 +762,7 @@ __device__ __forceinline__ void order_pair(float& na, uint32_t& ea, float& nb, u
 template <int STACK>
 __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uint32_t e1, float n2, uint32_t e2,
                                             float n3, uint32_t e3, uint2 (&stack)[STACK], int& sp, uint32_t& cur,
-                                            uint32_t& cur_count) {
+                                            uint32_t& cur_count, float& cur_near) {
     order_pair(n0, e0, n1, e1);
     order_pair(n2, e2, n3, e3);
     order_pair(n0, e0, n2, e2);
@@ -752,6 +776,7 @@ __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uin
     if (n1 != INFINITY) stack[sp++] = make_uint2(e1, __float_as_uint(n1));
     cur = e0 & kRefMask;
     cur_count = e0 >> kLeafShift;
+    cur_near = n0;
     return 1;
 }
 
@@ -764,9 +789,11 @@ __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uin
 // rays the occluder reported may differ, visibility does not.  Half as many
 // dependent node fetches per ray as the child-pair layout, each twice as
 // wide.
-template <bool ANY, bool COUNT, int STACK, bool C = false>
+template <bool ANY, bool COUNT, int STACK, bool C = false, bool CONTEST = false>
 __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const TraceRay& ray,
-                                               const TraceOptions& opt, TraceCounters* cnt) {
+                                               const TraceOptions& opt, TraceCounters* cnt,
+                                               bool* contested = nullptr) {
+    static_assert(!(CONTEST && (ANY || C)), "a contest is a matter of exact closest hits");
     TraceHit h;
     h.t = ray.tmax;
     h.u = 0.0f;
@@ -778,6 +805,7 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
         h.status = 1u;
         return h;
     }
+    if (CONTEST) *contested = false;
     if (s.wide_count == 0u) return h;
     using S = SlabOf<C>;
     const typename S::Ray sr = S::make(ray);
@@ -796,6 +824,8 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
     float lim = S::limit(ray.tmax, sr);  // what box near distances are compared against
     uint32_t best_i = 0xffffffffu, best_p = 0xffffffffu;
     uint32_t cur = 0u, cur_count = 0u;
+    float cur_near = 0.0f;                          // of the box being visited
+    bool rival = false, tied = false, late = false;  // CONTEST, see reach
     uint32_t steps = 0u;
     const uint32_t max_steps = s.wide_count * 5u + 8u;
     while (true) {
@@ -821,9 +851,10 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
             S::planes4(sr, pl, lim, n);
             // Entered children have finite near distances (near < tMax);
             // the others sort last at +inf.
-            const int down =
-                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
+            const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
+                                                 cur_count, cur_near);
             if (down < 0) {
+                if (CONTEST) *contested = true;
                 h.status = 2u;
                 h.tri = 0xffffffffu;
                 return h;
@@ -854,6 +885,7 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
                 if ((flags & kTriAlphaMask) != 0u) {
                     const int acc = alpha_accept(s.alpha, ti, u, v);
                     if (acc < 0) {
+                        if (CONTEST) *contested = true;
                         h.status = 3u;
                         h.tri = 0xffffffffu;
                         return h;
@@ -863,6 +895,23 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
                 if (ANY) {
                     h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
                     return h;
+                }
+                if constexpr (CONTEST) {
+                    // lim and limit_cmp reach past the best hit: a second hit
+                    // this near rivals it, a nearer one beyond its reach
+                    // settles what was rivalled behind it.
+                    const float to = reach(t);
+                    tied = found && (t == limit || (tied && t > limit));
+                    rival = found && (t >= limit || limit < to);
+                    if (!found || t < limit) {
+                        found = true;
+                        limit = t;
+                        limit_cmp = fminf(to, ray.tmax);
+                        lim = limit_cmp;
+                        late = cur_near > t;
+                        h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
+                    }
+                    continue;
                 }
                 const bool lower_key = t == limit && (key.x < best_i || (key.x == best_i && key.y < best_p));
                 if (!found || t < limit || lower_key) {
@@ -884,11 +933,13 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
             if (pn >= lim) continue;
             cur = e.x & kRefMask;
             cur_count = e.x >> kLeafShift;
+            cur_near = pn;
             next = true;
             break;
         }
         if (!next) break;
     }
+    if (CONTEST) *contested = tied || (rival && late);
     return h;
 }
 
@@ -1178,8 +1229,9 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
             // As in trace_wide.
             float n[4];
             S::planes4(sr, pl, lim, n);
-            const int down =
-                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
+            float unused;
+            const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
+                                                 cur_count, unused);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;
@@ -1238,6 +1290,165 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
             }
             leaf_count = 0u;
         }
+    }
+    return h;
+}
+
+// Four-wide traversal of one ray by a whole warp, for queues too short to give
+// every lane of the device a ray: there a kernel lasts as long as its slowest
+// ray, a chain of dependent node fetches, while most lanes idle.  The warp
+// keeps one stack in shared memory and takes up to eight entries off it at
+// once, four lanes to an entry: a lane tests one child box of a node or one
+// triangle of a leaf.  Boxes and triangles are tested with trace_wide's
+// arithmetic, so visibility is trace_wide's, and so is a closest hit that is
+// not contested (see reach).  Entries are pushed farthest first within a node,
+// the nodes in stack order.  Every lane passes the same ray, whose tMin is not
+// negative (distances compare as their bits), and gets the same hit.
+//
+// With at most kCoopBroad entries on the stack eight are taken, which leaves at
+// most kCoopBroad + 24; above it one at a time, which adds at most the tree's
+// depth-first bound (64 here): kCoopStack holds both.
+constexpr int kCoopBroad = 16;
+constexpr int kCoopStack = kCoopBroad + 24 + 64;
+
+template <bool ANY>
+__device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const TraceRay& ray, const TraceOptions& opt,
+                                               uint2* stack, bool& contested) {
+    contested = false;
+    TraceHit h;
+    h.t = ray.tmax;
+    h.u = 0.0f;
+    h.v = 0.0f;
+    h.tri = 0xffffffffu;
+    h.front = 0u;
+    h.status = 0u;
+    if (!ray_is_valid(ray)) {
+        h.status = 1u;
+        return h;
+    }
+    if (s.wide_count == 0u) return h;
+    const SlabRay sr = make_slab_ray(ray);
+    {
+        float root_near;
+        if (!slab_test(sr, s.root_lo[0], s.root_hi[0], s.root_lo[1], s.root_hi[1], s.root_lo[2], s.root_hi[2],
+                       ray.tmax, root_near))
+            return h;
+    }
+    const uint32_t lane = threadIdx.x & 31u, group = lane >> 2, child = lane & 3u;
+    // Offsets (in floats) of this lane's entry and exit planes in a node.
+    const uint32_t xn = (sr.neg_x ? 4u : 0u) + child, xf = (sr.neg_x ? 0u : 4u) + child;
+    const uint32_t yn = (sr.neg_y ? 12u : 8u) + child, yf = (sr.neg_y ? 8u : 12u) + child;
+    const uint32_t zn = (sr.neg_z ? 20u : 16u) + child, zf = (sr.neg_z ? 16u : 20u) + child;
+    float limit_cmp = ray.tmax;  // then the reach of the best hit
+    bool late = false;
+    int sp = 1;
+    if (lane == 0u) stack[0] = make_uint2(0u, 0u);
+    __syncwarp();
+    uint32_t steps = 0u;
+    const uint32_t max_steps = s.wide_count * 5u + 8u;
+    while (sp > 0) {
+        if (++steps > max_steps) {  // malformed (cyclic) tree guard
+            h.status = 3u;
+            h.tri = 0xffffffffu;
+            return h;
+        }
+        const int take = sp > kCoopBroad ? 1 : min(sp, 8);
+        uint32_t entry = 0u;
+        float box_near = 0.f;
+        bool live = int(group) < take;
+        if (live) {
+            const uint2 e = stack[sp - 1 - int(group)];
+            entry = e.x;
+            box_near = __uint_as_float(e.y);
+            live = box_near < limit_cmp;
+        }
+        const uint32_t cur = entry & kRefMask, count = entry >> kLeafShift;
+        float near_t = INFINITY;  // of an entered child
+        uint32_t child_entry = 0u;
+        float t = INFINITY, u = 0.f, v = 0.f;  // of this lane's nearest triangle hit
+        uint32_t tri = 0xffffffffu;
+        bool front = false, lane_contested = false, bad = false;
+        if (live && count == 0u) {
+            const float* w = reinterpret_cast<const float*>(s.wide + size_t(cur) * 8u);
+            child_entry = __ldg(reinterpret_cast<const uint32_t*>(w) + 24u + child);
+            float nn;
+            // An empty slot's +inf box is never entered.
+            if (slab_test_planes(sr, __ldg(w + xn), __ldg(w + xf), __ldg(w + yn), __ldg(w + yf), __ldg(w + zn),
+                                 __ldg(w + zf), limit_cmp, nn))
+                near_t = nn;
+        } else if (live) {
+            for (uint32_t k = child; k < count; k += 4u) {
+                const uint32_t ti = cur + k;
+                const float4* tp = s.tris + size_t(ti) * 4u;
+                const float4 p0 = __ldg(tp + 0), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
+                if (__float_as_uint(e1.w) == opt.ignore_instance && __float_as_uint(e2.w) == opt.ignore_primitive)
+                    continue;
+                const uint32_t flags = __float_as_uint(p0.w);
+                if (opt.shadow && (flags & kTriCastsShadow) == 0u) continue;
+                float tt, tu, tv;
+                bool tf;
+                if (!tri_test(ray, p0, e1, e2, limit_cmp, tt, tu, tv, tf)) continue;
+                if (!tf && (flags & kTriDoubleSided) == 0u) continue;
+                if ((flags & kTriAlphaMask) != 0u) {
+                    const int acc = alpha_accept(s.alpha, ti, tu, tv);
+                    bad |= acc < 0;
+                    if (acc <= 0) continue;
+                }
+                if (tri != 0xffffffffu) lane_contested = tt >= t ? lane_contested || tt < reach(t) : t < reach(tt);
+                if (tri != 0xffffffffu && tt >= t) continue;
+                t = tt; u = tu; v = tv; tri = ti; front = tf;
+            }
+        }
+        const uint32_t hits = __ballot_sync(0xffffffffu, tri != 0xffffffffu);
+        if (__any_sync(0xffffffffu, bad)) {
+            contested = true;
+            h.status = 3u;
+            h.tri = 0xffffffffu;
+            return h;
+        }
+        if (hits != 0u) {
+            const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(t)));
+            const int from = __ffs(__ballot_sync(0xffffffffu, t == best) & hits) - 1;
+            const float to = reach(best);
+            const bool held = h.tri != 0xffffffffu;
+            if (ANY) {
+                h.t = best;
+                h.tri = __shfl_sync(0xffffffffu, tri, from);
+                return h;
+            }
+            if (held && best >= h.t) {
+                contested = contested || late || best == h.t;
+            } else {
+                late = __shfl_sync(0xffffffffu, box_near > t ? 1u : 0u, from) != 0u;
+                const bool rival = (held && h.t < to) || __popc(__ballot_sync(0xffffffffu, t < to)) > 1 ||
+                                   __any_sync(0xffffffffu, lane_contested && t < to);
+                contested = rival && (late || __popc(__ballot_sync(0xffffffffu, t == best)) > 1 ||
+                                      __any_sync(0xffffffffu, lane_contested && t == best));
+                h.t = best;
+                h.u = __shfl_sync(0xffffffffu, u, from);
+                h.v = __shfl_sync(0xffffffffu, v, from);
+                h.tri = __shfl_sync(0xffffffffu, tri, from);
+                h.front = __shfl_sync(0xffffffffu, front ? 1u : 0u, from);
+                limit_cmp = fminf(to, ray.tmax);
+            }
+        }
+        // Entered children go back in place of what was taken.
+        const bool entered = near_t < limit_cmp;
+        const uint32_t mask = __ballot_sync(0xffffffffu, entered);
+        const float n1 = __shfl_xor_sync(0xffffffffu, near_t, 1), n2 = __shfl_xor_sync(0xffffffffu, near_t, 2),
+                    n3 = __shfl_xor_sync(0xffffffffu, near_t, 3);
+        if (entered) {
+            // Entered children of this node that are farther (equal: the later
+            // child), then those of nodes that were lower on the stack.
+            auto farther = [&](float n, uint32_t x) {
+                return n < limit_cmp && (n > near_t || (n == near_t && (child ^ x) > child)) ? 1u : 0u;
+            };
+            const uint32_t below = lane < 28u ? __popc(mask >> ((group + 1u) * 4u)) : 0u;
+            const uint32_t at = uint32_t(sp - take) + below + farther(n1, 1u) + farther(n2, 2u) + farther(n3, 3u);
+            stack[at] = make_uint2(child_entry, __float_as_uint(near_t));
+        }
+        sp += __popc(mask) - take;
+        __syncwarp();
     }
     return h;
 }
@@ -1433,8 +1644,9 @@ struct WideTraverser {
             const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
             float n[4];
             slab_test_planes4(sr, pl, limit_cmp, n);
-            const int down =
-                wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur, cur_count);
+            float unused;
+            const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
+                                                 cur_count, unused);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;

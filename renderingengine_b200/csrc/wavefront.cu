@@ -156,16 +156,26 @@ __device__ __forceinline__ TraceHit trace_mode(const TraceSceneView& s, const Tr
     return trace<ANY, COUNT, STACK>(s, ray, opt, cnt);
 }
 
-template <int STACK, int MODE = 0>
-__device__ __forceinline__ float4 intersect_one(const SceneSlot& sc, float4 o, float4 dir) {
-    TraceRay ray{from4(o), from4(dir), o.w, dir.w};
-    TraceOptions opt{kInv, kInv, false};
-    const TraceHit h = trace_mode<false, false, STACK, MODE>(sc.scene, ray, opt, nullptr);
+__device__ __forceinline__ float4 encode_hit(const TraceHit& h) {
     uint32_t code = h.tri;
     if (h.status != 0u) code = 0xfffffffeu;  // invalid ray / malformed: error hit
     else if (h.tri != kInv) code = h.tri | (h.front ? 0x80000000u : 0u);
     return make_float4(h.t, h.u, h.v, __uint_as_float(code));
 }
+
+template <int STACK, int MODE = 0>
+__device__ __forceinline__ float4 intersect_one(const SceneSlot& sc, float4 o, float4 dir) {
+    TraceRay ray{from4(o), from4(dir), o.w, dir.w};
+    TraceOptions opt{kInv, kInv, false};
+    return encode_hit(trace_mode<false, false, STACK, MODE>(sc.scene, ray, opt, nullptr));
+}
+
+// Queues up to this many rays per resident warp are traced a ray per warp
+// (trace_coop).  Swept in factors of two over whole frames: an 801x449 frame
+// went from 1,246 us to 1,110 at 2 and 1,097 at 4 and 8, a 256x256 Cornell
+// frame from 417 to 381 at 2 and 417 at 8, a 720p ReSTIR frame from 4,174 to
+// 4,086 at 2 and 4,183 at 8; a 1080p frame's tails are longer than that.
+constexpr uint32_t kCoopRaysPerWarp = 2u;
 
 // 1024 threads per SM (at most 64 registers): traversal is issue-bound and
 // wants every warp the register file allows.  The CTA size (128, 256 or 512
@@ -175,11 +185,30 @@ template <int STACK, int MODE, int BLOCK = 128>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_intersect(WfDevice d, uint32_t bounce) {
     const uint32_t q = bounce & 1u;
     const uint32_t count = *slot(d, bounce, kSlotRays);
-    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkIntersect))) {
-        const uint32_t i = w.item();
+    constexpr bool kCoop = STACK == 64 && (MODE == 2 || MODE == 4);
+    __shared__ uint2 stacks[kCoop ? BLOCK / 32 : 1][kCoop ? kCoopStack : 1];
+    const bool coop = kCoop && count <= kCoopRaysPerWarp * gridDim.x * (BLOCK / 32);
+    for (WarpWork w(count, 1u, coop ? 1u : 32u); w.more(); w.next(slot(d, bounce, kSlotWorkIntersect))) {
+        uint32_t i = w.item();
+        if constexpr (kCoop) {
+            if (coop) {
+                const float4 o = d.ray_o[q][w.base], dir = d.ray_d[q][w.base];
+                bool contested;
+                const TraceHit h = trace_coop<false>(d.scenes[d.ray_path[q][w.base] >> kPathBits].scene,
+                                                     TraceRay{from4(o), from4(dir), o.w, dir.w},
+                                                     TraceOptions{kInv, kInv, false}, stacks[threadIdx.x >> 5],
+                                                     contested);
+                // A contested hit is left to the loop below, on one lane.
+                if (!contested) {
+                    if (i < count) d.hit[i] = encode_hit(h);
+                    i = count;
+                }
+            }
+        }
         if (i < count)
             d.hit[i] = intersect_one<STACK, MODE>(d.scenes[d.ray_path[q][i] >> kPathBits], d.ray_o[q][i],
                                                   d.ray_d[q][i]);
+        __syncwarp();
     }
 }
 
@@ -221,13 +250,6 @@ __global__ void __launch_bounds__(128) k_intersect_counted(WfDevice d, uint32_t 
         }
         add_tests(cnt + bounce * 3u, c);
     }
-}
-
-__device__ __forceinline__ float4 encode_hit(const TraceHit& h) {
-    uint32_t code = h.tri;
-    if (h.status != 0u) code = 0xfffffffeu;
-    else if (h.tri != kInv) code = h.tri | (h.front ? 0x80000000u : 0u);
-    return make_float4(h.t, h.u, h.v, __uint_as_float(code));
 }
 
 // Persistent Intersect with per-lane refill: a lane whose ray finished takes
@@ -1392,65 +1414,6 @@ __global__ void __launch_bounds__(128, MINB) k_shade_b_capped(WfDevice d, uint32
 // ---------------------------------------------------------------------------
 // TraceShadow (TraceShadow.hlsl:5-92), Physical shadow method.
 // ---------------------------------------------------------------------------
-// One shadow query; returns the traversal tests through `c` when counting.
-template <int STACK, bool COUNT, int MODE = 0>
-__device__ __forceinline__ void shadow_one(const WfDevice& d, uint32_t bounce, uint32_t i, TraceCounters* c) {
-    const float4 o = d.sh_o[i];
-    const float4 dir = d.sh_d[i];
-    const uint4 sid = d.sh_id[i];
-    const uint32_t p = sid.x & kPathMask;
-    const SceneSlot& sc = d.scenes[sid.x >> kPathBits];
-    if (p >= d.capacity) {
-        set_fatal(d, kFatalShadePathIndex);
-        return;
-    }
-    TraceRay ray{from4(o), from4(dir), o.w, dir.w};
-    // Exclude the sampled light's own (instance, primitive), as the
-    // megakernel's PbrEvaluateShadowVisibilityL6 does
-    // (pbr_megakernel.hlsl:178-186): with a normal-offset origin and
-    // tMax = distance - epsilon the ray otherwise meets the light itself.
-    uint32_t ign_inst = kInv;
-    if (sid.z < sc.lights.light_count)
-        ign_inst = __ldg(reinterpret_cast<const uint4*>(sc.lights.lights + size_t(sid.z) * 6u + 5)).w;
-    TraceOptions opt{ign_inst, sid.w, true};
-    const TraceHit h = trace_mode<true, COUNT, STACK, MODE>(sc.scene, ray, opt, c);
-    if (h.status != 0u) {
-        atomicAdd(slot(d, bounce, kSlotNonFinite), 1u);
-        uint4 id = d.ident[p];
-        id.w = (id.w & ~kPathActive) | kPathTerminated | kPathError;
-        d.ident[p] = id;
-        return;
-    }
-    if (h.tri != kInv) return;  // occluded
-    const f3 cd = from4(d.sh_cd[i]);
-    const f3 cs = from4(d.sh_cs[i]);
-    float4* dp = sid.y == 0u ? d.acc_dd : d.acc_id;
-    float4* sp = sid.y == 0u ? d.acc_ds : d.acc_is;
-    const f3 df = from4(dp[p]) + cd;
-    const f3 sf = from4(sp[p]) + cs;
-    if (!finite_nonneg3(df) || !finite_nonneg3(sf)) {
-        atomicAdd(slot(d, bounce, kSlotNonFinite), 1u);
-        uint4 id = d.ident[p];
-        id.w = (id.w & ~kPathActive) | kPathTerminated | kPathError;
-        d.ident[p] = id;
-        return;
-    }
-    dp[p] = to4(df, 0.f);
-    sp[p] = to4(sf, 0.f);
-}
-
-template <int STACK, bool COUNT, int MODE = 0, int BLOCK = 128>
-__global__ void __launch_bounds__(BLOCK, COUNT ? 1 : 1024 / BLOCK) k_shadow(WfDevice d, uint32_t bounce,
-                                                                            unsigned long long* cnt) {
-    const uint32_t count = min(*slot(d, bounce, kSlotShadows), d.capacity);
-    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkShadow))) {
-        const uint32_t i = w.item();
-        TraceCounters c{};
-        if (i < count) shadow_one<STACK, COUNT, MODE>(d, bounce, i, &c);
-        if (COUNT) add_tests(cnt + 3u * kMaxDepth + bounce * 3u, c);
-    }
-}
-
 // Accumulates a finished shadow query into its path (TraceShadow.hlsl:33-92).
 __device__ __forceinline__ void shadow_finish(const WfDevice& d, uint32_t bounce, uint32_t i, const TraceHit& h) {
     const uint4 sid = d.sh_id[i];
@@ -1478,6 +1441,67 @@ __device__ __forceinline__ void shadow_finish(const WfDevice& d, uint32_t bounce
     }
     dp[p] = to4(df, 0.f);
     sp[p] = to4(sf, 0.f);
+}
+
+// Ray and rules of shadow query i; false when its path index is out of range.
+__device__ __forceinline__ bool shadow_setup(const WfDevice& d, uint32_t i, TraceRay& ray, TraceOptions& opt,
+                                             const SceneSlot*& sc) {
+    const float4 o = d.sh_o[i];
+    const float4 dir = d.sh_d[i];
+    const uint4 sid = d.sh_id[i];
+    sc = d.scenes + (sid.x >> kPathBits);
+    if ((sid.x & kPathMask) >= d.capacity) {
+        set_fatal(d, kFatalShadePathIndex);
+        return false;
+    }
+    ray = TraceRay{from4(o), from4(dir), o.w, dir.w};
+    // Exclude the sampled light's own (instance, primitive), as the
+    // megakernel's PbrEvaluateShadowVisibilityL6 does
+    // (pbr_megakernel.hlsl:178-186): with a normal-offset origin and
+    // tMax = distance - epsilon the ray otherwise meets the light itself.
+    uint32_t ign_inst = kInv;
+    if (sid.z < sc->lights.light_count)
+        ign_inst = __ldg(reinterpret_cast<const uint4*>(sc->lights.lights + size_t(sid.z) * 6u + 5)).w;
+    opt = TraceOptions{ign_inst, sid.w, true};
+    return true;
+}
+
+// One shadow query; returns the traversal tests through `c` when counting.
+template <int STACK, bool COUNT, int MODE = 0>
+__device__ __forceinline__ void shadow_one(const WfDevice& d, uint32_t bounce, uint32_t i, TraceCounters* c) {
+    TraceRay ray;
+    TraceOptions opt;
+    const SceneSlot* sc;
+    if (shadow_setup(d, i, ray, opt, sc))
+        shadow_finish(d, bounce, i, trace_mode<true, COUNT, STACK, MODE>(sc->scene, ray, opt, c));
+}
+
+template <int STACK, bool COUNT, int MODE = 0, int BLOCK = 128>
+__global__ void __launch_bounds__(BLOCK, COUNT ? 1 : 1024 / BLOCK) k_shadow(WfDevice d, uint32_t bounce,
+                                                                            unsigned long long* cnt) {
+    const uint32_t count = min(*slot(d, bounce, kSlotShadows), d.capacity);
+    if constexpr (!COUNT && STACK == 64 && (MODE == 2 || MODE == 4)) {
+        __shared__ uint2 stacks[BLOCK / 32][kCoopStack];
+        const uint32_t warps = gridDim.x * (BLOCK / 32);
+        if (count <= kCoopRaysPerWarp * warps) {
+            for (uint32_t i = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < count; i += warps) {
+                TraceRay ray;
+                TraceOptions opt;
+                const SceneSlot* sc;
+                if (!shadow_setup(d, i, ray, opt, sc)) continue;
+                bool contested;  // visibility never is
+                const TraceHit h = trace_coop<true>(sc->scene, ray, opt, stacks[threadIdx.x >> 5], contested);
+                if ((threadIdx.x & 31) == 0) shadow_finish(d, bounce, i, h);
+            }
+            return;
+        }
+    }
+    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkShadow))) {
+        const uint32_t i = w.item();
+        TraceCounters c{};
+        if (i < count) shadow_one<STACK, COUNT, MODE>(d, bounce, i, &c);
+        if (COUNT) add_tests(cnt + 3u * kMaxDepth + bounce * 3u, c);
+    }
 }
 
 // TraceShadow with per-lane refill (see k_intersect_refill).
