@@ -1601,6 +1601,7 @@ namespace {
 
 constexpr uint32_t kMaxViews = RE_MAX_BATCH_VIEWS;
 constexpr uint32_t kFrameRing = 4;
+constexpr uint32_t kThreeKernelPixels = 1u << 18;
 // One frame record: the batch header followed by up to kMaxViews views.
 constexpr size_t kFrameRecordBytes = sizeof(BatchParams) + size_t(kMaxViews) * sizeof(FrameParams);
 
@@ -1634,6 +1635,8 @@ struct re_renderer {
     int device = 0;
     uint32_t max_w = 0, max_h = 0, max_depth = 0, capacity = 0;
     re_renderer_tuning tuning{128, 0, 0, 1, 4, 0, 3};  // split inlined Shade, traversal chosen per launch
+    bool shade_by_launch = true;  // no tuning set: two or three Shade kernels by the launch's size
+    uint32_t batch_shade = 4;     // the staged launch's Shade variant
     re_scene* scene = nullptr;  // scene of slot 0 (the single-view API)
     SlotState slots[kMaxSceneSlots];
     uint32_t generation_counter = 0;
@@ -1966,7 +1969,7 @@ cudaError_t record_frame_t(re_renderer* r, uint32_t depth, cudaStream_t s, const
     const bool fuse = r->tuning.fuse_intersect_shade != 0 && hk.cnt == nullptr && hk.ev == nullptr;
     for (uint32_t b = 0; b < depth; ++b) {
         if (fuse) {
-            launch_shade<true, STACK>(r->tuning.shade_variant, grid_for, s, d, b);
+            launch_shade<true, STACK>(r->batch_shade, grid_for, s, d, b);
         } else {
             if (hk.cnt != nullptr && r->batch_eight != 0u) {
                 auto ki = r->batch_eight == 6u ? k_intersect_counted<STACK, 6> : k_intersect_counted<STACK, 5>;
@@ -2004,7 +2007,7 @@ cudaError_t record_frame_t(re_renderer* r, uint32_t depth, cudaStream_t s, const
                 launch_intersect_tb<STACK, 0>(tb, grid_tb, s, d, b);
             }
             mark();
-            launch_shade<false, STACK>(r->tuning.shade_variant, grid_for, s, d, b);
+            launch_shade<false, STACK>(r->batch_shade, grid_for, s, d, b);
         }
         mark();
         if (hk.cnt != nullptr && r->batch_eight != 0u) {
@@ -2304,11 +2307,12 @@ re_status stage_views(re_renderer* r, const re_view_desc* views, uint32_t n, uin
     if (r->ring_used[ring]) RE_CUDA_TRY(cudaEventSynchronize(r->ring_done[ring]));
     char* rec = r->host_frame + size_t(ring) * kFrameRecordBytes;
     FrameParams* fps = reinterpret_cast<FrameParams*>(rec + sizeof(BatchParams));
-    uint32_t pixel_total = 0;
+    uint32_t pixel_total = 0, shade_pixels = 0;
     for (uint32_t k = 0; k < n; ++k) {
         fill_view(r, views[order[k]], profile, fps[k]);
         fps[k].pixel_base = pixel_total;
         pixel_total += fps[k].pixel_count;
+        if (fps[k].rs.enabled == 0u) shade_pixels += fps[k].pixel_count;
     }
     BatchParams bp{n, path_end, depth, profile, pixel_total, 0u, 0u, 0u};
     std::memcpy(rec, &bp, sizeof(bp));
@@ -2316,6 +2320,13 @@ re_status stage_views(re_renderer* r, const re_view_desc* views, uint32_t n, uin
                                 cudaMemcpyHostToDevice, s));
     RE_CUDA_TRY(cudaEventRecord(r->ring_done[ring], s));
     r->ring_used[ring] = true;
+    // Until a tuning is set, launches with enough pixels whose direct light the
+    // Shade stage samples run it as three kernels, so NEE runs on surviving
+    // vertices only, and smaller ones as two, saving a kernel per bounce.
+    // Three kernels against two: 1280x720 heightfield 1,813 / 1,863 us a frame,
+    // 1280x720 soup 2,169 / 2,245, 256x256 Cornell 343 / 321; the lines cross
+    // between 200,000 and 330,000 pixels.
+    r->batch_shade = r->shade_by_launch && shade_pixels >= kThreeKernelPixels ? 5u : r->tuning.shade_variant;
     r->restir_active = restir;
     r->batch_deep_binary = deep;
     r->batch_wide = wide;
@@ -2333,7 +2344,7 @@ re_status launch_staged(re_renderer* r, cudaStream_t s) {
     RE_CUDA_TRY(cudaEventRecord(r->ev0, s));
     const uint64_t key = (uint64_t(depth) << 4) ^ (frame_stack_deep(r) ? 1 : 0) ^ (r->restir_active ? 2 : 0) ^
                          (r->batch_wide ? 4 : 0) ^ (r->batch_deep_binary ? 8 : 0) ^
-                         (uint64_t(r->batch_loop) << 32);
+                         (uint64_t(r->batch_loop) << 32) ^ (uint64_t(r->batch_shade) << 40);
     if (r->tuning.use_graph) {
         auto it = std::find_if(r->graphs.begin(), r->graphs.end(),
                                [key](const std::pair<uint64_t, cudaGraphExec_t>& g) { return g.first == key; });
@@ -2501,6 +2512,7 @@ RE_API re_status re_renderer_set_tuning(re_renderer* r, const re_renderer_tuning
     if (t->shade_variant > 7) return set_error(RE_INVALID_ARGUMENT, "shade variant must be 0 to 7");
     if (t->traversal_mode > 8) return set_error(RE_INVALID_ARGUMENT, "traversal mode must be 0 to 8");
     r->tuning = *t;
+    r->shade_by_launch = false;
     drop_graph(r);
     return clear_error();
 }
