@@ -922,6 +922,61 @@ re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth)
     return RE_SUCCESS;
 }
 
+namespace {
+
+// Quad node of every child-pair node (trace_quad_any): its grandchildren, or a
+// child itself where that is a leaf.
+__global__ void k_quad_nodes(const DeviceNode* nodes, uint32_t count, WideNode* quads) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const DeviceNode nd = nodes[i];
+    float lo[3][4], hi[3][4];
+    uint32_t entry[4];
+    auto put = [&](int slot, const DeviceNode& d, int side) {
+        lo[0][slot] = side == 0 ? d.a[0] : d.b[2]; hi[0][slot] = side == 0 ? d.a[1] : d.b[3];
+        lo[1][slot] = side == 0 ? d.a[2] : d.c[0]; hi[1][slot] = side == 0 ? d.a[3] : d.c[1];
+        lo[2][slot] = side == 0 ? d.b[0] : d.c[2]; hi[2][slot] = side == 0 ? d.b[1] : d.c[3];
+        entry[slot] = d.d[side] | (d.d[2 + side] << kWideLeafShift);
+    };
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        if (nd.d[2 + side] == 0u) {
+            const DeviceNode c = nodes[nd.d[side]];
+            put(2 * side, c, 0);
+            put(2 * side + 1, c, 1);
+        } else {
+            put(2 * side, nd, side);
+            for (int a = 0; a < 3; ++a) {
+                lo[a][2 * side + 1] = INFINITY;
+                hi[a][2 * side + 1] = -INFINITY;
+            }
+            entry[2 * side + 1] = kWideEmpty;
+        }
+    }
+    float4* o = reinterpret_cast<float4*>(quads + i);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        o[2 * a] = make_float4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
+        o[2 * a + 1] = make_float4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
+    }
+    reinterpret_cast<uint4*>(o)[6] = make_uint4(entry[0], entry[1], entry[2], entry[3]);
+    reinterpret_cast<uint4*>(o)[7] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+}  // namespace
+
+// Makes the scene's quad nodes; false when it has no memory for them.
+bool make_quad_nodes(re_scene* sc, cudaStream_t stream) {
+    if (sc->quad_nodes.reserve(size_t(sc->device_node_count) * sizeof(WideNode)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    k_quad_nodes<<<(sc->device_node_count + 127u) / 128u, 128, 0, stream>>>(
+        static_cast<const DeviceNode*>(sc->nodes.ptr), sc->device_node_count,
+        static_cast<WideNode*>(sc->quad_nodes.ptr));
+    return cudaStreamSynchronize(stream) == cudaSuccess;  // later batches may use any stream
+}
+
 // The scene from CanonicalTraversalTriangle records in device memory: the
 // checks, the LBVH passes, the leaf-ordered records and the four-wide nodes,
 // all on the device; the host reads the flags and bounds once and the wide

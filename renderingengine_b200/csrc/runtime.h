@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -76,6 +77,8 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
 // `scratch` (wide_scratch_bytes of the child-pair node count).
 size_t wide_scratch_bytes(uint32_t interior);
 re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth);
+// Quad nodes of the scene's child pairs (traverse.cuh, trace_quad_any).
+bool make_quad_nodes(re_scene* sc, cudaStream_t stream);
 // Fills sc->flat's nodes and leaf order when the tree was built on the device.
 re_status host_flat(const re_scene* sc);
 // Child-pair device nodes of sc->flat.
@@ -130,6 +133,11 @@ struct re_scene {
     re::DeviceBuffer stage_rays{true};
     re::DeviceBuffer stage_hits{true};
     re::DeviceBuffer work_counter{true};
+    // Quad nodes of any-hit batches, made with the first batch that walks them
+    // (quad_state: 0 not asked for, 1 there, 2 no memory).
+    re::DeviceBuffer quad_nodes{true};
+    std::mutex quad_mutex;
+    std::atomic<int> quad_state{0};
     re::DeviceBuffer counters{true};
     // Four-wide nodes over the same triangles (re::WideNode): made with the
     // scene for this library's own trees, else on first use by a renderer

@@ -234,6 +234,7 @@ struct BatchArgs {
     float4* hits;         // re_hit_record as 6 x float4
     uint32_t count;
     uint32_t* work;       // persistent work counter
+    const float4* quads;  // any-hit over quad nodes
     unsigned long long* counters;  // 9 slots (re_traversal_counters order)
 };
 
@@ -308,6 +309,22 @@ __global__ void __launch_bounds__(128, WIDE ? 8 : 1) trace_batch_kernel(BatchArg
     }
 }
 
+// Any-hit batch over the quad nodes: trace_batch_kernel<true, false>'s hits from
+// half the dependent node fetches.  400,009 random rays over 60,000 triangles:
+// 668 us over the child pairs, 529 here; bound by instruction issue.
+template <int STACK>
+__global__ void __launch_bounds__(128, 8) trace_quad_kernel(BatchArgs args) {
+    for (WarpWork w(args.count); w.more(); w.next(args.work)) {
+        const uint32_t i = w.item();
+        if (i >= args.count) continue;
+        uint4 ident;
+        const TraceRay ray = batch_ray(args, i, ident);
+        const TraceHit h =
+            trace_quad_any<STACK>(args.scene, args.quads, ray, TraceOptions{kInvalid, kInvalid, false});
+        write_hit_record(args.view, ray, h, ident, args.hits + size_t(i) * 6u);
+    }
+}
+
 // CTAs of `kernel` (128 threads) that fit on the device at once; a fact of the
 // kernel and the device, looked up once per device.
 template <auto K>
@@ -340,21 +357,57 @@ cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t str
 
 // Closest-hit batches over the four-wide nodes: on the library's own trees (in
 // a caller's flattened nodes a child box may stick out of its parent's, and the
-// child-pair loop tests every box on the way down) of enough triangles, with
-// enough rays to fill the device.  1.5 million rays over 36 triangles: 107 / 315
-// us (camera / random) over the four-wide nodes against 92 / 259 over the child
-// pairs; over 60,000 the four-wide nodes are 13 % faster for random rays.
-constexpr uint32_t kWideTraceTriangles = 1u << 14, kWideTraceRays = 1u << 16;
+// child-pair loop tests every box on the way down) of enough triangles.
+// 1,048,576 random rays, four-wide / child pairs: soups of 1,000 triangles 370 /
+// 392 us, 4,000 465 / 506, 16,000 976 / 1,134, 60,000 1,385 / 1,639; 500 rays
+// 21 / 23, 25 / 31, 43 / 49, 70 / 80.  Over the 36 triangles of a Cornell box
+// camera rays take 76 / 68, and over 1,000 triangles 96 / 94.
+constexpr uint32_t kWideTraceTriangles = 1u << 12;
+bool trace_over_wide(const re_scene* sc) {
+    return sc->own_tree && sc->triangle_count >= kWideTraceTriangles && sc->wide_node_count != 0u &&
+           sc->wide_stack_bound <= 64u && sc->flat.max_depth <= 64u;
+}
 
-bool trace_over_wide(const re_scene* sc, uint32_t count) {
-    return sc->own_tree && sc->triangle_count >= kWideTraceTriangles && count >= kWideTraceRays &&
-           sc->wide_node_count != 0u && sc->wide_stack_bound <= 64u && sc->flat.max_depth <= 64u;
+// Any-hit batches over the quad nodes, on the library's own trees by the same
+// reasoning, where the scene has quad nodes.  They are made, once, by the first
+// batch (not being captured) that by itself gains what they cost, a pass over
+// the nodes of about 30 us for 606,208 triangles and a few launches' time:
+// 262,144 random rays, quad nodes / child pairs: soups of 1,000 triangles 101 /
+// 117 us, 16,000 274 / 337, 60,000 383 / 477, the 606,208 145 / 171 (camera rays
+// 182 / 254).  With the nodes there 500 rays take 19 / 23, 39 / 50, 64 / 80 and
+// 33 / 46.
+constexpr uint32_t kQuadMakingRays = 1u << 18;
+const float4* quad_nodes(re_scene* sc, uint32_t count, cudaStream_t stream) {
+    if (!sc->own_tree || sc->layout_meta.root_is_leaf != 0u || sc->flat.max_depth > 64u) return nullptr;
+    if (sc->quad_state.load(std::memory_order_acquire) == 0 && count >= kQuadMakingRays &&
+        count >= sc->triangle_count / 2u) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        std::lock_guard<std::mutex> lock(sc->quad_mutex);
+        if (sc->quad_state.load(std::memory_order_relaxed) == 0) {
+            // Another thread may be capturing a stream of its own.
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            sc->quad_state.store(make_quad_nodes(sc, stream) ? 1 : 2, std::memory_order_release);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+        }
+    }
+    return sc->quad_state.load(std::memory_order_acquire) == 1 ? static_cast<const float4*>(sc->quad_nodes.ptr)
+                                                               : nullptr;
 }
 
 template <bool ANY, bool COUNT>
 cudaError_t launch_batch(re_scene* sc, BatchArgs args, cudaStream_t stream) {
+    if constexpr (ANY && !COUNT) {
+        // Three entries a node of two levels stay within 96 + 3 for 64 levels.
+        args.quads = quad_nodes(sc, args.count, stream);
+        if (args.quads != nullptr) return launch_batch_k<trace_quad_kernel<100>>(sc, args, stream);
+    }
     if constexpr (!ANY && !COUNT) {
-        if (trace_over_wide(sc, args.count))
+        if (trace_over_wide(sc))
             return launch_batch_k<trace_batch_kernel<false, false, 64, true>>(sc, args, stream);
     }
     if (sc->flat.max_depth <= 64) return launch_batch_k<trace_batch_kernel<ANY, COUNT, 64, false>>(sc, args, stream);
@@ -386,7 +439,7 @@ re_status run_trace_chunked(re_scene* sc, const re_trace_batch* b, cudaStream_t 
     const uint32_t n = b->ray_count;
     RE_CUDA_TRY(sc->stage_rays.reserve(size_t(n) * sizeof(re_ray_record)));
     RE_CUDA_TRY(sc->stage_hits.reserve(size_t(n) * sizeof(re_hit_record)));
-    RE_CUDA_TRY(sc->work_counter.reserve(2 * sizeof(uint32_t)));
+    RE_CUDA_TRY(sc->work_counter.reserve(sizeof(uint32_t)));
     if (sc->copy_in == nullptr) {
         RE_CUDA_TRY(cudaStreamCreateWithFlags(&sc->copy_in, cudaStreamNonBlocking));
         RE_CUDA_TRY(cudaStreamCreateWithFlags(&sc->copy_out, cudaStreamNonBlocking));
@@ -423,6 +476,7 @@ re_status run_trace_chunked(re_scene* sc, const re_trace_batch* b, cudaStream_t 
         args.count = cnt;
         args.work = static_cast<uint32_t*>(sc->work_counter.ptr);
         args.counters = nullptr;
+        args.quads = nullptr;
         if (!ok(launch_batch<ANY, false>(sc, args, stream)) || !ok(cudaEventRecord(run[k], stream)) ||
             !ok(cudaStreamWaitEvent(sc->copy_out, run[k], 0)))
             break;
@@ -459,7 +513,7 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
         d_rays = static_cast<const re_ray_record*>(sc->stage_rays.ptr);
         d_hits = static_cast<re_hit_record*>(sc->stage_hits.ptr);
     }
-    RE_CUDA_TRY(sc->work_counter.reserve(2 * sizeof(uint32_t)));
+    RE_CUDA_TRY(sc->work_counter.reserve(sizeof(uint32_t)));
     BatchArgs args;
     args.scene = scene_view(sc);
     args.view.attrs = static_cast<const float4*>(sc->attrs.ptr);
@@ -469,6 +523,7 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
     args.count = b->ray_count;
     args.work = static_cast<uint32_t*>(sc->work_counter.ptr);
     args.counters = nullptr;
+    args.quads = nullptr;
     cudaError_t e;
     if (out_counters != nullptr) {
         RE_CUDA_TRY(sc->counters.reserve(9 * sizeof(unsigned long long)));
@@ -524,6 +579,12 @@ re_status upload_scene_nodes(re_scene* sc) {
     sc->root_hi[0] = r.bounds_max.x; sc->root_hi[1] = r.bounds_max.y; sc->root_hi[2] = r.bounds_max.z;
     sc->flat_node_count = uint32_t(sc->flat.nodes.size());
     return RE_SUCCESS;
+}
+
+// So that no batch of the scene has to reserve it, not one being captured either;
+// without it the first batch tries again and reports the failure.
+void reserve_work_counter(re_scene* sc) {
+    if (sc->work_counter.reserve(sizeof(uint32_t)) != cudaSuccess) cudaGetLastError();
 }
 
 // Four-wide nodes of a tree built on the host.  Without the memory for them
@@ -733,6 +794,7 @@ RE_API re_status re_scene_create(const re_scene_desc* desc, re_scene** out_scene
         delete sc;
         return st;
     }
+    reserve_work_counter(sc);
     sc->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     *out_scene = sc;
     return clear_error();
@@ -766,6 +828,7 @@ RE_API re_status re_scene_create_from_device(const re_scene_desc* desc, re_scene
         delete sc;
         return st;
     }
+    reserve_work_counter(sc);
     sc->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     *out_scene = sc;
     return clear_error();

@@ -58,10 +58,10 @@ struct Request {
 };
 
 // Device bytes a resident scene is charged: child-pair nodes, triangles and
-// attributes (re_scene_info.device_bytes without the four-wide nodes, which
-// have never been part of the charge) plus the renderer's per-slot tables.
+// attributes plus the renderer's per-slot tables.  (The four-wide nodes and the
+// build's leaf order have never been part of the charge.)
 uint64_t scene_bytes(const SceneRecord& rec, const re_scene_info& info) {
-    return info.device_bytes - rec.scene->wide_nodes.bytes + uint64_t(rec.tris.size()) * 4u +
+    return info.device_bytes - rec.scene->wide_nodes.bytes - rec.scene->leaf_order.bytes + uint64_t(rec.tris.size()) * 4u +
            rec.materials.size() * sizeof(re_material) + rec.lights.size() * (sizeof(re_light) + 24u) +
            rec.fixtures.size() * sizeof(re_float4);
 }

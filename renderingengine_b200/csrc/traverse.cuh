@@ -944,6 +944,146 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
 }
 
 // ---------------------------------------------------------------------------
+// Any-hit traversal two levels of the child-pair tree at a time, in `trace`'s
+// order.  A quad node (WideNode's layout, one per child-pair node) holds the
+// four grandchildren: slots 0 and 1 the left child's children, 2 and 3 the
+// right's; a child that is a leaf takes its pair's first slot, and an empty slot
+// has lo = +inf and hi = -inf, whose entry distance is +inf and exit -inf for
+// either direction sign.  A child's box is the union of its children's, and
+// (plane - o) * inv is monotonic in the plane, rounding included, so the
+// child's entry distance per axis is the smaller of its children's, and a
+// grandchild that is entered has an entered parent: the nearer pair first, the
+// nearer of a pair first, left on equal, is the order in which `trace` reaches
+// them, and the occluder found is `trace`'s.  (A NaN distance -- origin on a
+// plane of a zero direction component -- is no constraint in `trace` and stays
+// NaN, hence ignored, in min.NaN.)  The distance limit of an any-hit ray does
+// not move, so what is pushed early is not pruned differently.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+template <int STACK>
+__device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, const float4* quads, const TraceRay& ray,
+                                                   const TraceOptions& opt) {
+    TraceHit h;
+    h.t = ray.tmax;
+    h.u = 0.0f;
+    h.v = 0.0f;
+    h.tri = 0xffffffffu;
+    h.front = 0u;
+    h.status = 0u;
+    if (!ray_is_valid(ray)) {
+        h.status = 1u;
+        return h;
+    }
+    if (s.node_count == 0u) return h;
+    const SlabRay sr = make_slab_ray(ray);
+    {
+        float root_near;
+        if (!slab_test(sr, s.root_lo[0], s.root_hi[0], s.root_lo[1], s.root_hi[1], s.root_lo[2], s.root_hi[2],
+                       ray.tmax, root_near))
+            return h;
+    }
+    uint32_t stack[STACK];
+    int sp = 0;
+    uint32_t cur = 0u, cur_count = 0u;
+    uint32_t steps = 0u;
+    const uint32_t max_steps = s.node_count * 4u + 8u;
+    while (true) {
+        if (++steps > max_steps) {  // malformed (cyclic) tree guard
+            h.status = 3u;
+            h.tri = 0xffffffffu;
+            return h;
+        }
+        if (cur_count == 0u) {
+            const float4* w = quads + size_t(cur) * 8u;
+            const WidePlanes p = load_wide_planes(w, sr);
+            const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
+            const float2 nx0 = plane_pair(p.xn.x, p.xn.y, sr.o.x, sr.inv.x), nx1 = plane_pair(p.xn.z, p.xn.w, sr.o.x, sr.inv.x);
+            const float2 fx0 = plane_pair(p.xf.x, p.xf.y, sr.o.x, sr.inv.x), fx1 = plane_pair(p.xf.z, p.xf.w, sr.o.x, sr.inv.x);
+            const float2 ny0 = plane_pair(p.yn.x, p.yn.y, sr.o.y, sr.inv.y), ny1 = plane_pair(p.yn.z, p.yn.w, sr.o.y, sr.inv.y);
+            const float2 fy0 = plane_pair(p.yf.x, p.yf.y, sr.o.y, sr.inv.y), fy1 = plane_pair(p.yf.z, p.yf.w, sr.o.y, sr.inv.y);
+            const float2 nz0 = plane_pair(p.zn.x, p.zn.y, sr.o.z, sr.inv.z), nz1 = plane_pair(p.zn.z, p.zn.w, sr.o.z, sr.inv.z);
+            const float2 fz0 = plane_pair(p.zf.x, p.zf.y, sr.o.z, sr.inv.z), fz1 = plane_pair(p.zf.z, p.zf.w, sr.o.z, sr.inv.z);
+            auto max3 = [](float a, float b, float c) {
+                float r;
+                asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+                return r;
+            };
+            auto child = [&](float nx, float ny, float nz, float fx, float fy, float fz) {
+                const float tn = max3(nx, ny, nz);
+                float tf;
+                asm("min.f32 %0, %1, %2, %3;" : "=f"(tf) : "f"(fx), "f"(fy), "f"(fz));
+                return !(tf < tn) && tf > sr.tmin && tn < ray.tmax ? fmaxf(tn, sr.tmin) : INFINITY;
+            };
+            float n0 = child(nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x);
+            float n1 = child(nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y);
+            float n2 = child(nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x);
+            float n3 = child(nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y);
+            const float nl = fmaxf(max3(min_nan(nx0.x, nx0.y), min_nan(ny0.x, ny0.y), min_nan(nz0.x, nz0.y)), sr.tmin);
+            const float nr = fmaxf(max3(min_nan(nx1.x, nx1.y), min_nan(ny1.x, ny1.y), min_nan(nz1.x, nz1.y)), sr.tmin);
+            uint32_t e0 = ent.x, e1 = ent.y, e2 = ent.z, e3 = ent.w;
+            order_pair(n0, e0, n1, e1);
+            order_pair(n2, e2, n3, e3);
+            if (nr < nl) {
+                const float a = n0, b = n1;
+                const uint32_t c = e0, d = e1;
+                n0 = n2; n1 = n3; e0 = e2; e1 = e3;
+                n2 = a; n3 = b; e2 = c; e3 = d;
+            }
+            if (sp + 3 > STACK) {
+                h.status = 2u;
+                h.tri = 0xffffffffu;
+                return h;
+            }
+            // Entered children of a pair come first in it; last visited is
+            // pushed first.
+            if (n3 != INFINITY) stack[sp++] = e3;
+            if (n2 != INFINITY) stack[sp++] = e2;
+            if (n1 != INFINITY) stack[sp++] = e1;
+            if (n0 != INFINITY) {
+                cur = e0 & kRefMask;
+                cur_count = e0 >> kLeafShift;
+                continue;
+            }
+        } else {
+            for (uint32_t k = 0; k < cur_count; ++k) {
+                const uint32_t ti = cur + k;
+                const float4* tp = s.tris + size_t(ti) * 4u;
+                const float4 p0 = __ldg(tp + 0), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
+                if (__float_as_uint(e1.w) == opt.ignore_instance && __float_as_uint(e2.w) == opt.ignore_primitive)
+                    continue;
+                const uint32_t flags = __float_as_uint(p0.w);
+                if (opt.shadow && (flags & kTriCastsShadow) == 0u) continue;
+                float t, u, v;
+                bool front;
+                if (!tri_test(ray, p0, e1, e2, ray.tmax, t, u, v, front)) continue;
+                if (!front && (flags & kTriDoubleSided) == 0u) continue;
+                if ((flags & kTriAlphaMask) != 0u) {
+                    const int acc = alpha_accept(s.alpha, ti, u, v);
+                    if (acc < 0) {
+                        h.status = 3u;
+                        h.tri = 0xffffffffu;
+                        return h;
+                    }
+                    if (acc == 0) continue;
+                }
+                h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
+                return h;
+            }
+        }
+        if (sp == 0) break;
+        const uint32_t e = stack[--sp];
+        cur = e & kRefMask;
+        cur_count = e >> kLeafShift;
+    }
+    return h;
+}
+
+// ---------------------------------------------------------------------------
 // Eight-wide traversal (Wide8Node, or Wide8QNode with Q): one node fetch
 // tests up to eight child boxes -- the plain form reads the exact boxes (14
 // aligned 16-byte loads), the compressed form six 16-byte loads and decodes
