@@ -89,11 +89,11 @@ __device__ __forceinline__ uint32_t tiled_pixel(uint32_t local, uint32_t width, 
 __global__ void k_raygen(WfDevice d) {
     const BatchParams bp = *d.batch;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < bp.pixel_total; base += stride) {
-        const uint32_t c = base + threadIdx.x;
-        const bool live = c < bp.pixel_total;
-        const uint32_t q = warp_append(slot(d, 0, kSlotRays), live);
-        if (!live) continue;
+    // Every pixel gets a ray, so a ray's place in the queue is its launch index:
+    // no atomic, and the queue keeps the pixels' order.
+    if (blockIdx.x == 0u && threadIdx.x == 0u) *slot(d, 0, kSlotRays) = bp.pixel_total;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < bp.pixel_total; c += stride) {
+        const uint32_t q = c;
         const uint32_t v = launch_view(d.views, bp.view_count, c);
         const FrameParams& fp = d.views[v];
         const uint32_t pix = tiled_pixel(c - fp.pixel_base, fp.width, fp.height);
