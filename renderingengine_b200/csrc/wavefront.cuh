@@ -30,7 +30,9 @@ constexpr uint32_t kRsStatGenerated = 0, kRsStatValid = 1, kRsStatRejected = 2, 
                    kRsStatTemporalAttempts = 4, kRsStatTemporalAccepted = 5, kRsStatSpatialAttempts = 6,
                    kRsStatSpatialAccepted = 7, kRsStatVisSubmitted = 8, kRsStatVisEvaluated = 9,
                    kRsStatVisVisible = 10, kRsStatVisDuplicate = 11;
-constexpr uint32_t kCounterWords = kGlobalBase + 16;
+// Work counters of the four ReSTIR kernels.
+constexpr uint32_t kSlotWorkRestir = kGlobalBase + 16;
+constexpr uint32_t kCounterWords = kGlobalBase + 20;
 
 // Path flags (WavefrontTypes.hlsli:42-50).
 constexpr uint32_t kPathActive = 1u << 0, kPathPrevDelta = 1u << 1, kPathPrevSpecular = 1u << 2,
@@ -163,7 +165,7 @@ struct WfDevice {
 
 // ReSTIR passes between the bounce loop and Resolve (restir.cu); grid-stride
 // over the batch's paths with `blocks` CTAs of 128 threads.
-void launch_restir(const WfDevice& d, uint32_t blocks, bool deep_stack, bool wide, cudaStream_t s);
+void launch_restir(const WfDevice& d, uint32_t sms, bool deep_stack, bool wide, cudaStream_t s);
 // RestirDebugV3 records (4 x uint4 per pixel) and view (float4 per pixel) of
 // `n` published reservoirs; either output may be null.
 void launch_restir_debug(const void* published, uint32_t n, uint32_t mode, uint32_t max_m, uint32_t max_age,
