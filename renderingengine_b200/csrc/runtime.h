@@ -118,6 +118,7 @@ struct re_scene {
     // The tree is this library's own (its child boxes lie in their parents'),
     // not the caller's flattened nodes.
     bool own_tree = true;
+    bool loose = false;  // some child box sticks out of its parent's
     re::DeviceLayout layout_meta;   // node_original / root flag (nodes freed after upload)
     // Resident device buffers.
     re::DeviceBuffer nodes{true};         // DeviceNode[]

@@ -132,6 +132,7 @@ TraceSceneView scene_view(const re_scene* sc) {
     v.alpha = static_cast<const AlphaView*>(sc->alpha_view.ptr);
     v.eight = static_cast<const float4*>(sc->eight_nodes.ptr);
     v.eightq = static_cast<const float4*>(sc->eight_qnodes.ptr);
+    v.loose = sc->loose ? 1u : 0u;
     v.eight_count = sc->eight_node_count;
     v.eight_stack = sc->eight_stack_bound;
     return v;
@@ -764,6 +765,13 @@ RE_API re_status re_scene_create(const re_scene_desc* desc, re_scene** out_scene
                 d[l.x] = d[l.z] = d[i] + 1;
             }
             depth = std::max(depth, d[i]);
+            for (uint32_t c : {l.x, l.z}) {
+                if (l.y != 0 || st != RE_SUCCESS) break;
+                const re_float4 &plo = desc->nodes[i].bounds_min, &phi = desc->nodes[i].bounds_max;
+                const re_float4 &clo = desc->nodes[c].bounds_min, &chi = desc->nodes[c].bounds_max;
+                sc->loose |= !(clo.x >= plo.x && clo.y >= plo.y && clo.z >= plo.z && chi.x <= phi.x &&
+                               chi.y <= phi.y && chi.z <= phi.z);
+            }
         }
         sc->flat.max_depth = depth;
         sc->flat.leaf_count = leaves;

@@ -50,6 +50,7 @@ struct TraceSceneView {
     const float4* eightq;    // Wide8QNode as 6 x float4 (null until built)
     uint32_t eight_count;
     uint32_t eight_stack;    // most stack entries an eight-wide traversal holds
+    uint32_t loose;          // some child box sticks out of its parent's (a caller's tree)
 };
 
 // A warp's share of a queue of `count` independent items in a persistent
@@ -75,6 +76,8 @@ struct WarpWork {
         const uint32_t lane = threadIdx.x & 31u;
         return lane < chunk && base + lane < count ? base + lane : count;
     }
+    // The next batch by number, without the counter.
+    __device__ __forceinline__ void skip() { base += warps * chunk; }
     __device__ __forceinline__ void next(uint32_t* work) {
         const uint32_t first = warps * chunk;
         if (first >= count) {  // every item was in a first batch
@@ -1441,7 +1444,8 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
 // once, four lanes to an entry: a lane tests one child box of a node or one
 // triangle of a leaf.  Boxes and triangles are tested with trace_wide's
 // arithmetic, so visibility is trace_wide's, and so is a closest hit that is
-// not contested (see reach).  Entries are pushed farthest first within a node,
+// not contested (see reach); an error is contested, another order may meet a hit
+// before it.  Entries are pushed farthest first within a node,
 // the nodes in stack order.  Every lane passes the same ray, whose tMin is not
 // negative (distances compare as their bits), and gets the same hit.
 //
@@ -1467,6 +1471,10 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
         return h;
     }
     if (s.wide_count == 0u) return h;
+    if (!ANY && s.loose != 0u) {  // there a hit may be pruned by a box above its leaf's
+        contested = true;
+        return h;
+    }
     const SlabRay sr = make_slab_ray(ray);
     {
         float root_near;

@@ -1480,26 +1480,29 @@ template <int STACK, bool COUNT, int MODE = 0, int BLOCK = 128>
 __global__ void __launch_bounds__(BLOCK, COUNT ? 1 : 1024 / BLOCK) k_shadow(WfDevice d, uint32_t bounce,
                                                                             unsigned long long* cnt) {
     const uint32_t count = min(*slot(d, bounce, kSlotShadows), d.capacity);
-    if constexpr (!COUNT && STACK == 64 && (MODE == 2 || MODE == 4)) {
-        __shared__ uint2 stacks[BLOCK / 32][kCoopStack];
-        const uint32_t warps = gridDim.x * (BLOCK / 32);
-        if (count <= kCoopRaysPerWarp * warps) {
-            for (uint32_t i = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < count; i += warps) {
+    constexpr bool kCoop = !COUNT && STACK == 64 && (MODE == 2 || MODE == 4);
+    __shared__ uint2 stacks[kCoop ? BLOCK / 32 : 1][kCoop ? kCoopStack : 1];
+    const bool coop = kCoop && count <= kCoopRaysPerWarp * gridDim.x * (BLOCK / 32);
+    for (WarpWork w(count, 1u, coop ? 1u : 32u); w.more();
+         coop ? w.skip() : w.next(slot(d, bounce, kSlotWorkShadow))) {
+        uint32_t i = w.item();
+        if constexpr (kCoop) {
+            if (coop) {
                 TraceRay ray;
                 TraceOptions opt;
                 const SceneSlot* sc;
-                if (!shadow_setup(d, i, ray, opt, sc)) continue;
-                bool contested;  // visibility never is
+                if (!shadow_setup(d, w.base, ray, opt, sc)) continue;
+                bool contested;
                 const TraceHit h = trace_coop<true>(sc->scene, ray, opt, stacks[threadIdx.x >> 5], contested);
-                if ((threadIdx.x & 31) == 0) shadow_finish(d, bounce, i, h);
+                if (!contested) {
+                    if (i < count) shadow_finish(d, bounce, i, h);
+                    i = count;
+                }
             }
-            return;
         }
-    }
-    for (WarpWork w(count); w.more(); w.next(slot(d, bounce, kSlotWorkShadow))) {
-        const uint32_t i = w.item();
         TraceCounters c{};
         if (i < count) shadow_one<STACK, COUNT, MODE>(d, bounce, i, &c);
+        __syncwarp();
         if (COUNT) add_tests(cnt + 3u * kMaxDepth + bounce * 3u, c);
     }
 }

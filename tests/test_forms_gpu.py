@@ -179,24 +179,55 @@ def _film(scene, data, w, h, depth, spp=1, **tuning):
     return r.read(FILM_SAMPLE, w * h).view(np.uint32)
 
 
-@pytest.mark.parametrize("build", [N.BUILD_FLATTENED_SAH, N.BUILD_LBVH], ids=["sah", "lbvh"])
-@pytest.mark.parametrize("w,h", [(1, 1), (33, 7), (97, 61)])
-def test_short_queues_equal_long_ones(native, w, h, build):
-    """A frame alone, its rays traced one per warp, against the same frame
-    beside one of a million pixels, traced 32 per warp; every surface, the
-    emitter's too, is there twice, so hits tie."""
+def _coincident():
     data = scenes.add_emissive_triangles(scenes.heightfield_scene(grid=48, spheres=48, seed=2), count=200, seed=5)
     data.triangles = _twice(data.triangles)
-    scene = Scene(data.triangles, data.fingerprint, 1, build)
+    return data
+
+
+def _unmasked():
+    """A tenth of the triangles alpha-masked without masks: rays that meet one
+    before a hit end in an error."""
+    data = scenes.add_emissive_triangles(scenes.heightfield_scene(grid=48, spheres=48, seed=2), count=200, seed=5)
+    data.triangles = data.triangles.copy()
+    data.triangles["metadata"][::10, 0] |= 2  # RE_GEOMETRY_FLAG_ALPHA_MASK
+    return data
+
+
+def _loose(data):
+    """The scene's flattened tree with every fifth box larger than its
+    parent's."""
+    nodes, order = Scene(data.triangles, data.fingerprint).export_flat()
+    nodes["bounds_min"][5::5, :3] -= 0.05
+    nodes["bounds_max"][5::5, :3] += 0.05
+    return Scene(np.ascontiguousarray(data.triangles[order]), data.fingerprint, 1, N.BUILD_FLATTENED_SAH, nodes=nodes)
+
+
+@pytest.mark.parametrize("make,build", [
+    (_coincident, lambda d: Scene(d.triangles, d.fingerprint)),
+    (_coincident, lambda d: Scene(d.triangles, d.fingerprint, 1, N.BUILD_LBVH)),
+    (_coincident, _loose),
+    (_unmasked, lambda d: Scene(d.triangles, d.fingerprint)),
+], ids=["sah", "lbvh", "loose", "unmasked"])
+@pytest.mark.parametrize("w,h", [(1, 1), (33, 7), (97, 61)])
+def test_short_queues_equal_long_ones(native, w, h, make, build):
+    """A frame alone, its rays traced one per warp, against the same frame
+    beside one of a million pixels, traced 32 per warp, where the order of
+    visits could show: every surface, the emitter's too, is there twice, or
+    masks are missing."""
+    data = make()
+    scene = build(data)
     for mode in (2, 4):
-        want = _film(scene, data, w, h, 8, traversal=mode)
-        r = Renderer(1280, 832, 8)
-        r.set_scene(scene, data)
-        r.set_tuning(traversal=mode)
-        r.render_views([dict(frame=frame_constants(data.camera, *size, 0, 8, seed=0x5151), offset=offset, key=offset)
-                        for size, offset in (((w, h), 0), ((1280, 800), w * h))])
-        assert r.collect().fatal_mask == 0
-        np.testing.assert_array_equal(r.read_view(FILM_SAMPLE, 0, w * h).view(np.uint32), want, err_msg=str(mode))
+        films = []
+        for others in ([], [((1280, 800), w * h)]):
+            r = Renderer(1280, 832, 8)
+            r.set_scene(scene, data)
+            r.set_tuning(traversal=mode)
+            r.render_views([dict(frame=frame_constants(data.camera, *size, 0, 8, seed=0x5151), offset=offset,
+                                 key=offset) for size, offset in [((w, h), 0)] + others])
+            assert r.collect().fatal_mask == 0
+            films.append(r.read_view(FILM_SAMPLE, 0, w * h).view(np.uint32))
+        np.testing.assert_array_equal(films[0], films[1], err_msg=str(mode))
 
 
 @pytest.mark.parametrize("w,h", [(511, 513), (512, 512), (1031, 257)])
