@@ -266,3 +266,24 @@ def test_atrous_row_blocks_match_oracle(native, oracle, w, h):
     ora = oracle.OracleSvgf(w, h, 2, native_cfg)
     for gb, sig, fi, trig in S.sequence(w, h, 3, 11, hostile=False):
         _compare(gpu.process(gb, sig, fi, trig), ora.process(gb, sig, fi, trig), f"frame {fi}")
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 1), (33, 7), (64, 4), (257, 3)])
+def test_export_to_any_word_address(native, w, h):
+    """Records written a warp at a time to addresses that only words align."""
+    import torch
+    data = scenes.heightfield_scene(grid=48, spheres=48, seed=2)
+    r = Renderer(w, h, 4)
+    r.set_scene(Scene(data.triangles, data.fingerprint), data)
+    fc = frame_constants(data.camera, w, h, 0, 4, seed=0x5151)
+    r.render(fc, accumulate=False)
+    r.collect()
+    want = r.export_reconstruction(fc, fc)
+    sizes = [w * h * N.GBUFFER_DTYPE.itemsize, w * h * N.SIGNAL_DTYPE.itemsize]
+    out = [torch.full((s + 32,), 0xA5, dtype=torch.uint8, device="cuda") for s in sizes]
+    r.export_reconstruction(fc, fc, gbuffer_ptr=out[0].data_ptr() + 4, signal_ptr=out[1].data_ptr() + 12)
+    torch.cuda.synchronize()
+    for buf, size, at, records in zip(out, sizes, (4, 12), want):
+        got = buf.cpu().numpy()
+        assert got[at:at + size].tobytes() == records.tobytes()
+        assert np.all(got[:at] == 0xA5) and np.all(got[at + size:] == 0xA5)
