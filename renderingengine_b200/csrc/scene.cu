@@ -132,7 +132,7 @@ TraceSceneView scene_view(const re_scene* sc) {
     v.alpha = static_cast<const AlphaView*>(sc->alpha_view.ptr);
     v.eight = static_cast<const float4*>(sc->eight_nodes.ptr);
     v.eightq = static_cast<const float4*>(sc->eight_qnodes.ptr);
-    v.loose = sc->loose ? 1u : 0u;
+    v.ordered = sc->loose || sc->alpha_masked ? 1u : 0u;
     v.eight_count = sc->eight_node_count;
     v.eight_stack = sc->eight_stack_bound;
     return v;
@@ -358,15 +358,16 @@ cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t str
 
 // Closest-hit batches over the four-wide nodes: on the library's own trees (in
 // a caller's flattened nodes a child box may stick out of its parent's, and the
-// child-pair loop tests every box on the way down) of enough triangles.
+// child-pair loop tests every box on the way down) of enough triangles, without
+// alpha masks (one that is missing is an error that another order may not meet).
 // 1,048,576 random rays, four-wide / child pairs: soups of 1,000 triangles 370 /
 // 392 us, 4,000 465 / 506, 16,000 976 / 1,134, 60,000 1,385 / 1,639; 500 rays
 // 21 / 23, 25 / 31, 43 / 49, 70 / 80.  Over the 36 triangles of a Cornell box
 // camera rays take 76 / 68, and over 1,000 triangles 96 / 94.
 constexpr uint32_t kWideTraceTriangles = 1u << 12;
 bool trace_over_wide(const re_scene* sc) {
-    return sc->own_tree && sc->triangle_count >= kWideTraceTriangles && sc->wide_node_count != 0u &&
-           sc->wide_stack_bound <= 64u && sc->flat.max_depth <= 64u;
+    return sc->own_tree && !sc->alpha_masked && sc->triangle_count >= kWideTraceTriangles &&
+           sc->wide_node_count != 0u && sc->wide_stack_bound <= 64u && sc->flat.max_depth <= 64u;
 }
 
 // Any-hit batches over the quad nodes, on the library's own trees by the same

@@ -50,7 +50,8 @@ struct TraceSceneView {
     const float4* eightq;    // Wide8QNode as 6 x float4 (null until built)
     uint32_t eight_count;
     uint32_t eight_stack;    // most stack entries an eight-wide traversal holds
-    uint32_t loose;          // some child box sticks out of its parent's (a caller's tree)
+    uint32_t ordered;        // the order of visits can decide a hit or an error: some child box sticks out
+                             // of its parent's (a caller's tree), or alpha masks that may be missing
 };
 
 // A warp's share of a queue of `count` independent items in a persistent
@@ -888,7 +889,6 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
                 if ((flags & kTriAlphaMask) != 0u) {
                     const int acc = alpha_accept(s.alpha, ti, u, v);
                     if (acc < 0) {
-                        if (CONTEST) *contested = true;
                         h.status = 3u;
                         h.tri = 0xffffffffu;
                         return h;
@@ -1444,8 +1444,9 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
 // once, four lanes to an entry: a lane tests one child box of a node or one
 // triangle of a leaf.  Boxes and triangles are tested with trace_wide's
 // arithmetic, so visibility is trace_wide's, and so is a closest hit that is
-// not contested (see reach); an error is contested, another order may meet a hit
-// before it.  Entries are pushed farthest first within a node,
+// not contested (see reach).  Scenes whose order of visits matters by itself are
+// contested whole: a hit may be pruned by a box above its leaf's, or an error be
+// met before the hit that ends another order.  Entries are pushed farthest first within a node,
 // the nodes in stack order.  Every lane passes the same ray, whose tMin is not
 // negative (distances compare as their bits), and gets the same hit.
 //
@@ -1471,7 +1472,7 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
         return h;
     }
     if (s.wide_count == 0u) return h;
-    if (!ANY && s.loose != 0u) {  // there a hit may be pruned by a box above its leaf's
+    if (s.ordered != 0u) {
         contested = true;
         return h;
     }
@@ -1515,7 +1516,7 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
         uint32_t child_entry = 0u;
         float t = INFINITY, u = 0.f, v = 0.f;  // of this lane's nearest triangle hit
         uint32_t tri = 0xffffffffu;
-        bool front = false, lane_contested = false, bad = false;
+        bool front = false, lane_contested = false;
         if (live && count == 0u) {
             const float* w = reinterpret_cast<const float*>(s.wide + size_t(cur) * 8u);
             child_entry = __ldg(reinterpret_cast<const uint32_t*>(w) + 24u + child);
@@ -1537,23 +1538,12 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
                 bool tf;
                 if (!tri_test(ray, p0, e1, e2, limit_cmp, tt, tu, tv, tf)) continue;
                 if (!tf && (flags & kTriDoubleSided) == 0u) continue;
-                if ((flags & kTriAlphaMask) != 0u) {
-                    const int acc = alpha_accept(s.alpha, ti, tu, tv);
-                    bad |= acc < 0;
-                    if (acc <= 0) continue;
-                }
                 if (tri != 0xffffffffu) lane_contested = tt >= t ? lane_contested || tt < reach(t) : t < reach(tt);
                 if (tri != 0xffffffffu && tt >= t) continue;
                 t = tt; u = tu; v = tv; tri = ti; front = tf;
             }
         }
         const uint32_t hits = __ballot_sync(0xffffffffu, tri != 0xffffffffu);
-        if (__any_sync(0xffffffffu, bad)) {
-            contested = true;
-            h.status = 3u;
-            h.tri = 0xffffffffu;
-            return h;
-        }
         if (hits != 0u) {
             const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(t)));
             const int from = __ffs(__ballot_sync(0xffffffffu, t == best) & hits) - 1;

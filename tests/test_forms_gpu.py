@@ -52,14 +52,17 @@ def _rays(tri, count, seed):
 
 
 @pytest.mark.parametrize("build", [N.BUILD_FLATTENED_SAH, N.BUILD_LBVH], ids=["sah", "lbvh"])
-@pytest.mark.parametrize("triangles,copies", [
-    (3, None), (9, None), (4095, None), (4096, None), (2048, 0), (8192, 0), (8192, 1), (8192, 3), (30000, 1)])
-def test_batch_forms_equal_child_pair_loop(native, build, triangles, copies):
+@pytest.mark.parametrize("triangles,copies,masked", [
+    (3, None, False), (9, None, False), (4095, None, False), (4096, None, False), (2048, 0, False), (8192, 0, False),
+    (8192, 1, False), (8192, 3, False), (30000, 1, False), (8192, None, True)])
+def test_batch_forms_equal_child_pair_loop(native, build, triangles, copies, masked):
     """Counted batches always walk the child pairs.  The quad nodes are there
     from the first any-hit batch of 2^18 rays on."""
     tri = scenes.triangle_soup(triangles, seed=triangles).triangles
     if copies is not None:
         tri = _twice(tri, copies)
+    if masked:  # without masks: an error for rays that meet one before a hit
+        tri["metadata"][::10, 0] |= 2  # RE_GEOMETRY_FLAG_ALPHA_MASK
     scene = Scene(tri, 5, 1, build)
     for count in (1, 333, (1 << 18) - 1, 1 << 18, 1, 333, 65569):
         rays = _rays(tri, count, seed=count)
