@@ -718,8 +718,9 @@ RE_API re_status re_renderer_restir_read(re_renderer* r, uint32_t plane, void* d
 /* Render server: continuous batching of render requests on one GPU.        */
 /* Requests (scene, camera, extent, depth, estimator incl. ReSTIR, samples) */
 /* arrive over time; every step renders one sample of every admitted        */
-/* request in batched launches (re_renderer_render_views; requests grouped  */
-/* by scene under a path budget, re_plan_launches), so requests             */
+/* request (a step of few paths renders further samples of requests without */
+/* temporal reuse) in batched launches (re_renderer_render_views; requests  */
+/* grouped by scene under a path budget, re_plan_launches), so requests     */
 /* that arrive while others are on the GPU join at the next step as path    */
 /* ranges and memory free up.  Scenes are registered once (host copies) and */
 /* made resident on demand with a GPU LBVH build; resident scenes, the path */
@@ -852,7 +853,7 @@ RE_API re_status re_bsdf_probe(const re_bsdf_query* queries, uint32_t count, re_
 /* ------------------------------------------------------------------------ */
 /* Allocation-free GPU LBVH build.  No counterpart in the reference: it is   */
 /* the GPU LBVH of re_scene_create(RE_BUILD_LBVH) (bounds, 30-bit Morton     */
-/* codes, stable radix sort on (code, stable ID), Karras hierarchy, refit)  */
+/* codes, stable radix sort on (code, stable ID), Karras hierarchy, boxes)  */
 /* for callers that cannot allocate device memory where they build, e.g. a  */
 /* renderer rebuilding small dynamic meshes between launches of a frame     */
 /* under a fixed memory budget, where a cudaMalloc would synchronise the    */
@@ -866,7 +867,7 @@ RE_API re_status re_bsdf_probe(const re_bsdf_query* queries, uint32_t count, re_
 /*     scratch address (cudaGetSymbolAddress); make it before any stream     */
 /*     capture.                                                             */
 /*   - No buffer needs to start at zero: each call re-initialises its own   */
-/*     bounds and refit counters.                                           */
+/*     bounds and counters.                                                 */
 /*   - The cached scratch address belongs to the device's context: a        */
 /*     cudaDeviceReset between calls is not supported (the next call would  */
 /*     launch on a stale address).                                          */

@@ -1,7 +1,7 @@
 """Render server: continuous batching of render requests (the C ABI's
 re_server_*).  Scenes are registered once as host records; requests arrive
-over time and are rendered one sample per launch together with every other
-admitted request, against an HBM budget with least-recently-used scene
+over time and are rendered a sample per step (more while a step is small)
+together with every other admitted request, against an HBM budget with least-recently-used scene
 eviction."""
 from __future__ import annotations
 
