@@ -30,6 +30,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "runtime.h"
@@ -223,6 +224,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     extern __shared__ __align__(16) unsigned char smem[];
     ClusterShared& S = *reinterpret_cast<ClusterShared*>(smem);
     cg::cluster_group cluster = cg::this_cluster();
+    // Another CTA's shared memory may only be accessed once that CTA has
+    // started, which a cluster barrier shows; the key loads cover its wait.
+    auto started = cluster.barrier_arrive();
     const uint32_t rank = cluster.block_rank(), t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     const uint32_t per = items * kClusterThreads;
     const uint32_t first = warp * 32u * items + lane;  // this lane's slots: first + 32 j
@@ -241,6 +245,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     atomicOr(&S.varying[0], __reduce_or_sync(0xffffffffu, uint32_t(vary)));
     atomicOr(&S.varying[1], __reduce_or_sync(0xffffffffu, uint32_t(vary >> 32)));
     __syncthreads();
+    cluster.barrier_wait(std::move(started));
     if (t < kClusterCtas)
         cluster.map_shared_rank(S.cta_varying, t)[rank] =
             (static_cast<unsigned long long>(S.varying[1]) << 32) | S.varying[0];
