@@ -929,7 +929,7 @@ re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth)
 
 namespace {
 
-// Quad node of every child-pair node (trace_quad_any): its grandchildren, or a
+// Quad node of every child-pair node (trace_quad): its grandchildren, or a
 // child itself where that is a leaf.
 __global__ void k_quad_nodes(const DeviceNode* nodes, uint32_t count, WideNode* quads) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

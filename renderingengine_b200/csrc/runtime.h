@@ -77,7 +77,7 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
 // `scratch` (wide_scratch_bytes of the child-pair node count).
 size_t wide_scratch_bytes(uint32_t interior);
 re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth);
-// Quad nodes of the scene's child pairs (traverse.cuh, trace_quad_any).
+// Quad nodes of the scene's child pairs (traverse.cuh, trace_quad).
 bool make_quad_nodes(re_scene* sc, cudaStream_t stream);
 // Fills sc->flat's nodes and leaf order when the tree was built on the device.
 re_status host_flat(const re_scene* sc);
@@ -134,7 +134,7 @@ struct re_scene {
     re::DeviceBuffer stage_rays{true};
     re::DeviceBuffer stage_hits{true};
     re::DeviceBuffer work_counter{true};
-    // Quad nodes of any-hit batches, made with the first batch that walks them
+    // Quad nodes of trace batches, made with the first batch that walks them
     // (quad_state: 0 not asked for, 1 there, 2 no memory).
     re::DeviceBuffer quad_nodes{true};
     std::mutex quad_mutex;

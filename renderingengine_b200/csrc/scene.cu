@@ -263,14 +263,6 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& c, unsigned 
     }
 }
 
-// Persistent traversal of a batch.  WIDE walks the four-wide nodes: half the
-// dependent node fetches of a ray and packed slab arithmetic, with the
-// child-pair loop's closest hit: contested rays (reach) are traced again over
-// the child pairs.  Any-hit batches, whose reported occluder is the first one
-// met, and the counting form keep the child pairs' visiting order.  Bound by
-// instruction issue and the dependent node fetches of a ray.  1080p camera rays
-// over 2,424,832 triangles: 754 us over the child pairs with 32-ray batches,
-// 712 with WarpWork, 633 over the four-wide nodes.
 __device__ __forceinline__ TraceRay batch_ray(const BatchArgs& args, uint32_t i, uint4& ident) {
     const float4* rp = args.rays + size_t(i) * 4u;
     const float4 ot = __ldg(rp + 0);
@@ -279,8 +271,9 @@ __device__ __forceinline__ TraceRay batch_ray(const BatchArgs& args, uint32_t i,
     return TraceRay{mk(ot.x, ot.y, ot.z), mk(dt.x, dt.y, dt.z), ot.w, dt.w};
 }
 
-template <bool ANY, bool COUNT, int STACK, bool WIDE>
-__global__ void __launch_bounds__(128, WIDE ? 8 : 1) trace_batch_kernel(BatchArgs args) {
+// Persistent traversal of a batch over the child pairs.
+template <bool ANY, bool COUNT, int STACK>
+__global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
     TraceOptions opt;
     opt.ignore_instance = kInvalid;
     opt.ignore_primitive = kInvalid;
@@ -291,14 +284,7 @@ __global__ void __launch_bounds__(128, WIDE ? 8 : 1) trace_batch_kernel(BatchArg
         if (i < args.count) {
             uint4 ident;
             const TraceRay ray = batch_ray(args, i, ident);
-            TraceHit h;
-            if constexpr (WIDE) {
-                bool contested;
-                h = trace_wide<false, false, STACK, false, true>(args.scene, ray, opt, nullptr, &contested);
-                if (contested) h = trace<false, false, STACK>(args.scene, ray, opt, nullptr);
-            } else {
-                h = trace<ANY, COUNT, STACK>(args.scene, ray, opt, &c);
-            }
+            const TraceHit h = trace<ANY, COUNT, STACK>(args.scene, ray, opt, &c);
             if (COUNT) {
                 if (h.status == 1u) atomicAdd(args.counters + 3, 1ull);
                 if (h.status == 2u) atomicAdd(args.counters + 2, 1ull);
@@ -310,18 +296,19 @@ __global__ void __launch_bounds__(128, WIDE ? 8 : 1) trace_batch_kernel(BatchArg
     }
 }
 
-// Any-hit batch over the quad nodes: trace_batch_kernel<true, false>'s hits from
-// half the dependent node fetches.  400,009 random rays over 60,000 triangles:
-// 668 us over the child pairs, 529 here; bound by instruction issue.
-template <int STACK>
+// Batch over the quad nodes: trace_batch_kernel<ANY, false>'s hits, in its order
+// of visits, from half the dependent node fetches.  2,073,600 closest-hit rays
+// over 2,424,832 triangles: camera rays 895 us over the child pairs, 814 here,
+// random rays 1,265 and 1,104; 400,009 random any-hit rays over 60,000
+// triangles: 668 and 529.
+template <bool ANY, int STACK>
 __global__ void __launch_bounds__(128, 8) trace_quad_kernel(BatchArgs args) {
     for (WarpWork w(args.count); w.more(); w.next(args.work)) {
         const uint32_t i = w.item();
         if (i >= args.count) continue;
         uint4 ident;
         const TraceRay ray = batch_ray(args, i, ident);
-        const TraceHit h =
-            trace_quad_any<STACK>(args.scene, args.quads, ray, TraceOptions{kInvalid, kInvalid, false});
+        const TraceHit h = trace_quad<ANY, STACK>(args.scene, args.quads, ray, TraceOptions{kInvalid, kInvalid, false});
         write_hit_record(args.view, ray, h, ident, args.hits + size_t(i) * 6u);
     }
 }
@@ -356,28 +343,17 @@ cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t str
     return cudaGetLastError();
 }
 
-// Closest-hit batches over the four-wide nodes: on the library's own trees (in
-// a caller's flattened nodes a child box may stick out of its parent's, and the
-// child-pair loop tests every box on the way down) of enough triangles, without
-// alpha masks (one that is missing is an error that another order may not meet).
-// 1,048,576 random rays, four-wide / child pairs: soups of 1,000 triangles 370 /
-// 392 us, 4,000 465 / 506, 16,000 976 / 1,134, 60,000 1,385 / 1,639; 500 rays
-// 21 / 23, 25 / 31, 43 / 49, 70 / 80.  Over the 36 triangles of a Cornell box
-// camera rays take 76 / 68, and over 1,000 triangles 96 / 94.
-constexpr uint32_t kWideTraceTriangles = 1u << 12;
-bool trace_over_wide(const re_scene* sc) {
-    return sc->own_tree && !sc->alpha_masked && sc->triangle_count >= kWideTraceTriangles &&
-           sc->wide_node_count != 0u && sc->wide_stack_bound <= 64u && sc->flat.max_depth <= 64u;
-}
-
-// Any-hit batches over the quad nodes, on the library's own trees by the same
-// reasoning, where the scene has quad nodes.  They are made, once, by the first
-// batch (not being captured) that by itself gains what they cost, a pass over
-// the nodes of about 30 us for 606,208 triangles and a few launches' time:
-// 262,144 random rays, quad nodes / child pairs: soups of 1,000 triangles 101 /
-// 117 us, 16,000 274 / 337, 60,000 383 / 477, the 606,208 145 / 171 (camera rays
-// 182 / 254).  With the nodes there 500 rays take 19 / 23, 39 / 50, 64 / 80 and
-// 33 / 46.
+// Batches over the quad nodes: on the library's own trees (in a caller's
+// flattened nodes a child's box need not be the union of its children's), where
+// the scene has quad nodes.  They are made, once, by the first batch (not being
+// captured) that by itself gains what they cost, a pass over the nodes of about
+// 30 us for 606,208 triangles and a few launches' time.  Random rays, quad nodes
+// / child pairs: 262,144 any-hit rays, soups of 1,000 triangles 101 / 117 us,
+// 16,000 274 / 337, 60,000 383 / 477, the 606,208 145 / 171 (camera rays 182 /
+// 254); closest hits 112 / 124, 297 / 355, 422 / 509, 167 / 191 (camera rays
+// 224 / 270).  With the nodes there 500 any-hit rays take 19 / 23, 39 / 50,
+// 64 / 80 and 33 / 46, closest 21 / 23, 41 / 52, 66 / 82 and 35 / 47.  Over the
+// 36 triangles of a Cornell box they are equal.
 constexpr uint32_t kQuadMakingRays = 1u << 18;
 const float4* quad_nodes(re_scene* sc, uint32_t count, cudaStream_t stream) {
     if (!sc->own_tree || sc->layout_meta.root_is_leaf != 0u || sc->flat.max_depth > 64u) return nullptr;
@@ -403,17 +379,13 @@ const float4* quad_nodes(re_scene* sc, uint32_t count, cudaStream_t stream) {
 
 template <bool ANY, bool COUNT>
 cudaError_t launch_batch(re_scene* sc, BatchArgs args, cudaStream_t stream) {
-    if constexpr (ANY && !COUNT) {
+    if constexpr (!COUNT) {
         // Three entries a node of two levels stay within 96 + 3 for 64 levels.
         args.quads = quad_nodes(sc, args.count, stream);
-        if (args.quads != nullptr) return launch_batch_k<trace_quad_kernel<100>>(sc, args, stream);
+        if (args.quads != nullptr) return launch_batch_k<trace_quad_kernel<ANY, 100>>(sc, args, stream);
     }
-    if constexpr (!ANY && !COUNT) {
-        if (trace_over_wide(sc))
-            return launch_batch_k<trace_batch_kernel<false, false, 64, true>>(sc, args, stream);
-    }
-    if (sc->flat.max_depth <= 64) return launch_batch_k<trace_batch_kernel<ANY, COUNT, 64, false>>(sc, args, stream);
-    return launch_batch_k<trace_batch_kernel<ANY, COUNT, 128, false>>(sc, args, stream);
+    if (sc->flat.max_depth <= 64) return launch_batch_k<trace_batch_kernel<ANY, COUNT, 64>>(sc, args, stream);
+    return launch_batch_k<trace_batch_kernel<ANY, COUNT, 128>>(sc, args, stream);
 }
 
 re_status validate_batch(const re_scene* sc, const re_trace_batch* b) {

@@ -16,6 +16,8 @@
 // of the node slab arithmetic can prune differently.
 #pragma once
 
+#include <type_traits>
+
 #include "device_math.cuh"
 #include "sah_builder.h"
 
@@ -766,7 +768,7 @@ __device__ __forceinline__ void order_pair(float& na, uint32_t& ea, float& nb, u
 template <int STACK>
 __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uint32_t e1, float n2, uint32_t e2,
                                             float n3, uint32_t e3, uint2 (&stack)[STACK], int& sp, uint32_t& cur,
-                                            uint32_t& cur_count, float& cur_near) {
+                                            uint32_t& cur_count) {
     order_pair(n0, e0, n1, e1);
     order_pair(n2, e2, n3, e3);
     order_pair(n0, e0, n2, e2);
@@ -780,7 +782,6 @@ __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uin
     if (n1 != INFINITY) stack[sp++] = make_uint2(e1, __float_as_uint(n1));
     cur = e0 & kRefMask;
     cur_count = e0 >> kLeafShift;
-    cur_near = n0;
     return 1;
 }
 
@@ -793,11 +794,9 @@ __device__ __forceinline__ int wide_descend(float n0, uint32_t e0, float n1, uin
 // rays the occluder reported may differ, visibility does not.  Half as many
 // dependent node fetches per ray as the child-pair layout, each twice as
 // wide.
-template <bool ANY, bool COUNT, int STACK, bool C = false, bool CONTEST = false>
+template <bool ANY, bool COUNT, int STACK, bool C = false>
 __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const TraceRay& ray,
-                                               const TraceOptions& opt, TraceCounters* cnt,
-                                               bool* contested = nullptr) {
-    static_assert(!(CONTEST && (ANY || C)), "a contest is a matter of exact closest hits");
+                                               const TraceOptions& opt, TraceCounters* cnt) {
     TraceHit h;
     h.t = ray.tmax;
     h.u = 0.0f;
@@ -809,7 +808,6 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
         h.status = 1u;
         return h;
     }
-    if (CONTEST) *contested = false;
     if (s.wide_count == 0u) return h;
     using S = SlabOf<C>;
     const typename S::Ray sr = S::make(ray);
@@ -828,8 +826,6 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
     float lim = S::limit(ray.tmax, sr);  // what box near distances are compared against
     uint32_t best_i = 0xffffffffu, best_p = 0xffffffffu;
     uint32_t cur = 0u, cur_count = 0u;
-    float cur_near = 0.0f;                          // of the box being visited
-    bool rival = false, tied = false, late = false;  // CONTEST, see reach
     uint32_t steps = 0u;
     const uint32_t max_steps = s.wide_count * 5u + 8u;
     while (true) {
@@ -856,9 +852,8 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
             // Entered children have finite near distances (near < tMax);
             // the others sort last at +inf.
             const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
-                                                 cur_count, cur_near);
+                                                 cur_count);
             if (down < 0) {
-                if (CONTEST) *contested = true;
                 h.status = 2u;
                 h.tri = 0xffffffffu;
                 return h;
@@ -899,23 +894,6 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
                     h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
                     return h;
                 }
-                if constexpr (CONTEST) {
-                    // lim and limit_cmp reach past the best hit: a second hit
-                    // this near rivals it, a nearer one beyond its reach
-                    // settles what was rivalled behind it.
-                    const float to = reach(t);
-                    tied = found && (t == limit || (tied && t > limit));
-                    rival = found && (t >= limit || limit < to);
-                    if (!found || t < limit) {
-                        found = true;
-                        limit = t;
-                        limit_cmp = fminf(to, ray.tmax);
-                        lim = limit_cmp;
-                        late = cur_near > t;
-                        h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
-                    }
-                    continue;
-                }
                 const bool lower_key = t == limit && (key.x < best_i || (key.x == best_i && key.y < best_p));
                 if (!found || t < limit || lower_key) {
                     found = true;
@@ -936,31 +914,34 @@ __device__ __forceinline__ TraceHit trace_wide(const TraceSceneView& s, const Tr
             if (pn >= lim) continue;
             cur = e.x & kRefMask;
             cur_count = e.x >> kLeafShift;
-            cur_near = pn;
             next = true;
             break;
         }
         if (!next) break;
     }
-    if (CONTEST) *contested = tied || (rival && late);
     return h;
 }
 
 // ---------------------------------------------------------------------------
-// Any-hit traversal two levels of the child-pair tree at a time, in `trace`'s
-// order.  A quad node (WideNode's layout, one per child-pair node) holds the
-// four grandchildren: slots 0 and 1 the left child's children, 2 and 3 the
-// right's; a child that is a leaf takes its pair's first slot, and an empty slot
-// has lo = +inf and hi = -inf, whose entry distance is +inf and exit -inf for
-// either direction sign.  A child's box is the union of its children's, and
+// Traversal two levels of the child-pair tree at a time, in `trace`'s order.  A
+// quad node (WideNode's layout, one per child-pair node) holds the four
+// grandchildren: slots 0 and 1 the left child's children, 2 and 3 the right's; a
+// child that is a leaf takes its pair's first slot, and an empty slot has
+// lo = +inf and hi = -inf, whose entry distance is +inf and exit -inf for either
+// direction sign.  A child's box is the union of its children's, and
 // (plane - o) * inv is monotonic in the plane, rounding included, so the
 // child's entry distance per axis is the smaller of its children's, and a
 // grandchild that is entered has an entered parent: the nearer pair first, the
 // nearer of a pair first, left on equal, is the order in which `trace` reaches
-// them, and the occluder found is `trace`'s.  (A NaN distance -- origin on a
-// plane of a zero direction component -- is no constraint in `trace` and stays
-// NaN, hence ignored, in min.NaN.)  The distance limit of an any-hit ray does
-// not move, so what is pushed early is not pruned differently.
+// them.  (A NaN distance -- origin on a plane of a zero direction component --
+// is no constraint in `trace` and stays NaN, hence ignored, in min.NaN.)  What is
+// pushed earlier than there is compared with the distance limit again when it is
+// popped, when `trace` would test it, and its child with a nearer box is not
+// pruned before it.  So the same triangles are tested in the same order against
+// the same limits, and the hit is `trace`'s whatever its distance's rounding.
+// That matters: a box starts at a distance that is accurate to a few ulps, but a
+// triangle's t is off by its conditioning, without bound for a ray along its
+// plane, so of two hits either can prune the other's box, and the first met wins.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float min_nan(float a, float b) {
     float r;
@@ -968,9 +949,9 @@ __device__ __forceinline__ float min_nan(float a, float b) {
     return r;
 }
 
-template <int STACK>
-__device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, const float4* quads, const TraceRay& ray,
-                                                   const TraceOptions& opt) {
+template <bool ANY, int STACK>
+__device__ __forceinline__ TraceHit trace_quad(const TraceSceneView& s, const float4* quads, const TraceRay& ray,
+                                               const TraceOptions& opt) {
     TraceHit h;
     h.t = ray.tmax;
     h.u = 0.0f;
@@ -990,8 +971,19 @@ __device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, cons
                        ray.tmax, root_near))
             return h;
     }
-    uint32_t stack[STACK];
+    // An any-hit ray's limit does not move: it needs no distances on the stack.
+    using Entry = std::conditional_t<ANY, uint32_t, uint2>;
+    Entry stack[STACK];
     int sp = 0;
+    bool found = false;
+    float limit = ray.tmax;
+    float limit_cmp = ray.tmax;  // see next_up
+    uint32_t best_i = 0xffffffffu, best_p = 0xffffffffu;
+    auto push = [&](float near_t, uint32_t e) {
+        if (near_t == INFINITY) return;
+        if constexpr (ANY) stack[sp++] = e;
+        else stack[sp++] = make_uint2(e, __float_as_uint(near_t));
+    };
     uint32_t cur = 0u, cur_count = 0u;
     uint32_t steps = 0u;
     const uint32_t max_steps = s.node_count * 4u + 8u;
@@ -1020,7 +1012,7 @@ __device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, cons
                 const float tn = max3(nx, ny, nz);
                 float tf;
                 asm("min.f32 %0, %1, %2, %3;" : "=f"(tf) : "f"(fx), "f"(fy), "f"(fz));
-                return !(tf < tn) && tf > sr.tmin && tn < ray.tmax ? fmaxf(tn, sr.tmin) : INFINITY;
+                return !(tf < tn) && tf > sr.tmin && tn < limit_cmp ? fmaxf(tn, sr.tmin) : INFINITY;
             };
             float n0 = child(nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x);
             float n1 = child(nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y);
@@ -1044,9 +1036,9 @@ __device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, cons
             }
             // Entered children of a pair come first in it; last visited is
             // pushed first.
-            if (n3 != INFINITY) stack[sp++] = e3;
-            if (n2 != INFINITY) stack[sp++] = e2;
-            if (n1 != INFINITY) stack[sp++] = e1;
+            push(n3, e3);
+            push(n2, e2);
+            push(n1, e1);
             if (n0 != INFINITY) {
                 cur = e0 & kRefMask;
                 cur_count = e0 >> kLeafShift;
@@ -1057,13 +1049,13 @@ __device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, cons
                 const uint32_t ti = cur + k;
                 const float4* tp = s.tris + size_t(ti) * 4u;
                 const float4 p0 = __ldg(tp + 0), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
-                if (__float_as_uint(e1.w) == opt.ignore_instance && __float_as_uint(e2.w) == opt.ignore_primitive)
-                    continue;
+                const uint2 key = make_uint2(__float_as_uint(e1.w), __float_as_uint(e2.w));
+                if (key.x == opt.ignore_instance && key.y == opt.ignore_primitive) continue;
                 const uint32_t flags = __float_as_uint(p0.w);
                 if (opt.shadow && (flags & kTriCastsShadow) == 0u) continue;
                 float t, u, v;
                 bool front;
-                if (!tri_test(ray, p0, e1, e2, ray.tmax, t, u, v, front)) continue;
+                if (!tri_test(ray, p0, e1, e2, limit_cmp, t, u, v, front)) continue;
                 if (!front && (flags & kTriDoubleSided) == 0u) continue;
                 if ((flags & kTriAlphaMask) != 0u) {
                     const int acc = alpha_accept(s.alpha, ti, u, v);
@@ -1074,14 +1066,38 @@ __device__ __forceinline__ TraceHit trace_quad_any(const TraceSceneView& s, cons
                     }
                     if (acc == 0) continue;
                 }
-                h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
-                return h;
+                if constexpr (ANY) {
+                    h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
+                    return h;
+                }
+                const bool lower_key = t == limit && (key.x < best_i || (key.x == best_i && key.y < best_p));
+                if (!found || t < limit || lower_key) {
+                    found = true;
+                    limit = t;
+                    limit_cmp = next_up(t);
+                    h.t = t; h.u = u; h.v = v; h.tri = ti; h.front = front ? 1u : 0u;
+                    best_i = key.x;
+                    best_p = key.y;
+                }
             }
         }
-        if (sp == 0) break;
-        const uint32_t e = stack[--sp];
-        cur = e & kRefMask;
-        cur_count = e >> kLeafShift;
+        // Pop the next entry that is still within the distance limit.
+        bool next = false;
+        while (sp > 0) {
+            uint32_t e;
+            if constexpr (ANY) {
+                e = stack[--sp];
+            } else {
+                const uint2 en = stack[--sp];
+                if (__uint_as_float(en.y) >= limit_cmp) continue;
+                e = en.x;
+            }
+            cur = e & kRefMask;
+            cur_count = e >> kLeafShift;
+            next = true;
+            break;
+        }
+        if (!next) break;
     }
     return h;
 }
@@ -1372,9 +1388,8 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
             // As in trace_wide.
             float n[4];
             S::planes4(sr, pl, lim, n);
-            float unused;
             const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
-                                                 cur_count, unused);
+                                                 cur_count);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;
@@ -1782,9 +1797,8 @@ struct WideTraverser {
             const uint4 ent = __ldg(reinterpret_cast<const uint4*>(w + 6));
             float n[4];
             slab_test_planes4(sr, pl, limit_cmp, n);
-            float unused;
             const int down = wide_descend<STACK>(n[0], ent.x, n[1], ent.y, n[2], ent.z, n[3], ent.w, stack, sp, cur,
-                                                 cur_count, unused);
+                                                 cur_count);
             if (down < 0) {
                 h.status = 2u;
                 h.tri = 0xffffffffu;
