@@ -382,20 +382,6 @@ __device__ __forceinline__ float next_up(float x) {
     return x >= 0.0f ? __uint_as_float((u & 0x7fffffffu) + 1u) : __uint_as_float(u - 1u);
 }
 
-// What makes a closest hit independent of the order of visits.  A box's near
-// distance and a triangle's t are rounded separately, so a box may start an
-// ulp or two behind the triangle in it; with another hit between the two, the
-// loop that meets the other one first prunes the box and the loop that meets
-// the box first does not.  A loop that must agree with another loop's order
-// therefore visits and tests up to `reach` of its best hit, 2^-16 beyond it
-// (a hundred times any such gap), and notes whether a second triangle was
-// hit within that margin.  If none was, every order of visits over the same leaf
-// boxes ends with this hit; also if the hit triangle's own box starts no later
-// than its t, since then no hit prunes it (and so between the two triangles of
-// a mesh edge).  Otherwise, or when two distances are equal, the hit is
-// `contested`, and the caller takes the other loop's.
-__device__ __forceinline__ float reach(float t) { return next_up(__fmaf_rn(fabsf(t), 0x1p-16f, t)); }
-
 // Moller-Trumbore in the CPU mirror's exact operation order.
 __device__ __forceinline__ bool tri_test(const TraceRay& r, float4 p0, float4 e1v, float4 e2v,
                                          float limit_cmp, float& t_out, float& u_out,
@@ -1457,21 +1443,38 @@ __device__ __forceinline__ TraceHit trace_wide_ww(const TraceSceneView& s, const
 // ray, a chain of dependent node fetches, while most lanes idle.  The warp
 // keeps one stack in shared memory and takes up to eight entries off it at
 // once, four lanes to an entry: a lane tests one child box of a node or one
-// triangle of a leaf.  Boxes and triangles are tested with trace_wide's
-// arithmetic, so visibility is trace_wide's, and so is a closest hit that is
-// not contested (see reach).  Scenes whose order of visits matters by itself are
-// contested whole: a hit may be pruned by a box above its leaf's, or an error be
-// met before the hit that ends another order.  Entries are pushed farthest first within a node,
-// the nodes in stack order.  Every lane passes the same ray, whose tMin is not
-// negative (distances compare as their bits), and gets the same hit.
+// triangle of a leaf.  Any hit ends an any-hit ray, whose limit does not move.
+//
+// A closest hit is the one that trace_wide finds, or with PARKED trace_wide_ww on
+// a warp of one ray, by that loop's order of visits: of two hits either can prune
+// the other's box (see trace_quad), so the order can decide.  The stack is in
+// that order, and so are the taken entries, the top one first.  They are settled
+// in turn up to the first node with children, which take its place.  What comes
+// after that stays, since hits in those children count first; only a later node
+// is replaced by its children already, ordered by wide_descend's network (which
+// orders those that the loop will still enter the same with or without the
+// others) and bounded by the hits before it, and dropped when it has none.
+// (A leaf's hit whose box does not start behind it bounds what follows: the leaf
+// is pruned only if the limit is below the hit already.)
+//
+// PARKED: trace_wide_ww takes the entry after a leaf off its stack before it
+// tests the leaf, so that entry is admitted by the limit before the leaf's hits.
+// A node uses that up, so one that is not settled yet leaves a mark before its
+// children (a node reference that no scene has).  On a warp of more rays that
+// loop postpones leaves for as long as another ray has none, so there the rays of
+// a warp decide such hits for one another.
+//
+// Scenes whose order of visits matters by itself (TraceSceneView::ordered) and
+// rays of a negative tMin are left to the caller (`contested`).  Every lane passes
+// the same ray and gets the same hit.
 //
 // With at most kCoopBroad entries on the stack eight are taken, which leaves at
-// most kCoopBroad + 24; above it one at a time, which adds at most the tree's
+// most kCoopBroad + 32; above it one at a time, which adds at most the tree's
 // depth-first bound (64 here): kCoopStack holds both.
 constexpr int kCoopBroad = 16;
-constexpr int kCoopStack = kCoopBroad + 24 + 64;
+constexpr int kCoopStack = kCoopBroad + 32 + 64;
 
-template <bool ANY>
+template <bool ANY, bool PARKED = false>
 __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const TraceRay& ray, const TraceOptions& opt,
                                                uint2* stack, bool& contested) {
     contested = false;
@@ -1487,7 +1490,7 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
         return h;
     }
     if (s.wide_count == 0u) return h;
-    if (s.ordered != 0u) {
+    if (s.ordered != 0u || !(ray.tmin >= 0.0f)) {
         contested = true;
         return h;
     }
@@ -1503,8 +1506,9 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
     const uint32_t xn = (sr.neg_x ? 4u : 0u) + child, xf = (sr.neg_x ? 0u : 4u) + child;
     const uint32_t yn = (sr.neg_y ? 12u : 8u) + child, yf = (sr.neg_y ? 8u : 12u) + child;
     const uint32_t zn = (sr.neg_z ? 20u : 16u) + child, zf = (sr.neg_z ? 16u : 20u) + child;
-    float limit_cmp = ray.tmax;  // then the reach of the best hit
-    bool late = false;
+    float limit_cmp = ray.tmax;  // see next_up
+    float admit = ray.tmax;      // the limit that admits the next entry
+    uint32_t best_i = 0xffffffffu, best_p = 0xffffffffu;
     int sp = 1;
     if (lane == 0u) stack[0] = make_uint2(0u, 0u);
     __syncwarp();
@@ -1517,22 +1521,20 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
             return h;
         }
         const int take = sp > kCoopBroad ? 1 : min(sp, 8);
-        uint32_t entry = 0u;
-        float box_near = 0.f;
+        uint2 e = make_uint2(0u, 0u);
         bool live = int(group) < take;
         if (live) {
-            const uint2 e = stack[sp - 1 - int(group)];
-            entry = e.x;
-            box_near = __uint_as_float(e.y);
-            live = box_near < limit_cmp;
+            e = stack[sp - 1 - int(group)];
+            live = __uint_as_float(e.y) < admit;
         }
-        const uint32_t cur = entry & kRefMask, count = entry >> kLeafShift;
+        const float box_near = __uint_as_float(e.y);
+        const uint32_t cur = e.x & kRefMask, count = e.x >> kLeafShift;
         float near_t = INFINITY;  // of an entered child
         uint32_t child_entry = 0u;
         float t = INFINITY, u = 0.f, v = 0.f;  // of this lane's nearest triangle hit
-        uint32_t tri = 0xffffffffu;
-        bool front = false, lane_contested = false;
-        if (live && count == 0u) {
+        uint32_t tri = 0xffffffffu, key_i = 0u, key_p = 0u;
+        bool front = false;
+        if (live && count == 0u && !(PARKED && cur == kRefMask)) {
             const float* w = reinterpret_cast<const float*>(s.wide + size_t(cur) * 8u);
             child_entry = __ldg(reinterpret_cast<const uint32_t*>(w) + 24u + child);
             float nn;
@@ -1540,67 +1542,121 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
             if (slab_test_planes(sr, __ldg(w + xn), __ldg(w + xf), __ldg(w + yn), __ldg(w + yf), __ldg(w + zn),
                                  __ldg(w + zf), limit_cmp, nn))
                 near_t = nn;
-        } else if (live) {
-            for (uint32_t k = child; k < count; k += 4u) {
+        } else {  // (no triangles: not live, or a mark)
+            for (uint32_t k = live ? child : count; k < count; k += 4u) {
                 const uint32_t ti = cur + k;
                 const float4* tp = s.tris + size_t(ti) * 4u;
                 const float4 p0 = __ldg(tp + 0), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
-                if (__float_as_uint(e1.w) == opt.ignore_instance && __float_as_uint(e2.w) == opt.ignore_primitive)
-                    continue;
+                const uint32_t ki = __float_as_uint(e1.w), kp = __float_as_uint(e2.w);
+                if (ki == opt.ignore_instance && kp == opt.ignore_primitive) continue;
                 const uint32_t flags = __float_as_uint(p0.w);
                 if (opt.shadow && (flags & kTriCastsShadow) == 0u) continue;
                 float tt, tu, tv;
                 bool tf;
                 if (!tri_test(ray, p0, e1, e2, limit_cmp, tt, tu, tv, tf)) continue;
                 if (!tf && (flags & kTriDoubleSided) == 0u) continue;
-                if (tri != 0xffffffffu) lane_contested = tt >= t ? lane_contested || tt < reach(t) : t < reach(tt);
-                if (tri != 0xffffffffu && tt >= t) continue;
+                if (tt > t || (tt == t && (ki > key_i || (ki == key_i && kp >= key_p)))) continue;
                 t = tt; u = tu; v = tv; tri = ti; front = tf;
+                key_i = ki; key_p = kp;
             }
         }
-        const uint32_t hits = __ballot_sync(0xffffffffu, tri != 0xffffffffu);
-        if (hits != 0u) {
-            const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(t)));
-            const int from = __ffs(__ballot_sync(0xffffffffu, t == best) & hits) - 1;
-            const float to = reach(best);
-            const bool held = h.tri != 0xffffffffu;
-            if (ANY) {
-                h.t = best;
-                h.tri = __shfl_sync(0xffffffffu, tri, from);
+        bool hit = tri != 0xffffffffu;
+        uint32_t hits = __ballot_sync(0xffffffffu, hit);
+        if constexpr (ANY) {
+            if (hits != 0u) {
+                h.t = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(t)));
+                h.tri = __shfl_sync(0xffffffffu, tri, __ffs(hits) - 1);
                 return h;
             }
-            if (held && best >= h.t) {
-                contested = contested || late || best == h.t;
-            } else {
-                late = __shfl_sync(0xffffffffu, box_near > t ? 1u : 0u, from) != 0u;
-                const bool rival = (held && h.t < to) || __popc(__ballot_sync(0xffffffffu, t < to)) > 1 ||
-                                   __any_sync(0xffffffffu, lane_contested && t < to);
-                contested = rival && (late || __popc(__ballot_sync(0xffffffffu, t == best)) > 1 ||
-                                      __any_sync(0xffffffffu, lane_contested && t == best));
-                h.t = best;
+        } else if ((hits & 0xeeeeeeeeu) != 0u) {
+            // The nearest of a leaf: lowest distance, key, place.
+#pragma unroll
+            for (int x = 1; x < 4; ++x) {
+                const float ot = __shfl_xor_sync(0xffffffffu, t, x);
+                const uint32_t oi = __shfl_xor_sync(0xffffffffu, key_i, x), op = __shfl_xor_sync(0xffffffffu, key_p, x),
+                               oti = __shfl_xor_sync(0xffffffffu, tri, x);
+                const bool less = oi != key_i ? oi < key_i : op != key_p ? op < key_p : oti < tri;
+                if (ot < t || (ot == t && less)) hit = false;
+            }
+            hits = __ballot_sync(0xffffffffu, hit);
+        }
+        uint32_t nodes = __ballot_sync(0xffffffffu, near_t != INFINITY);  // with children, by their lanes
+        uint32_t settled = nodes == 0u ? 32u : uint32_t(__ffs(nodes) - 1) & ~3u;  // lanes below hold settled entries
+        float bound = limit_cmp;  // the loop's limit, at most, when it comes to this lane's entry
+        if (!ANY && (hits != 0u || (PARKED && admit != limit_cmp))) {
+            // In turn.  (What the shortcut above settles otherwise changes nothing.)
+            settled = 32u;
+            for (uint32_t g = 0u; g < uint32_t(take) * 4u; g += 4u) {
+                const float bn = __shfl_sync(0xffffffffu, box_near, int(g));
+                if (!(bn < admit)) continue;
+                admit = limit_cmp;
+                if ((nodes >> g & 15u) != 0u) {
+                    nodes = __ballot_sync(0xffffffffu, near_t < limit_cmp);
+                    if ((nodes >> g & 15u) != 0u) {
+                        settled = g;
+                        break;
+                    }
+                }
+                const uint32_t from_hit = hits >> g & 15u;
+                if (from_hit == 0u) continue;
+                const int from = int(g) + __ffs(from_hit) - 1;
+                const float ct = __shfl_sync(0xffffffffu, t, from);
+                if (!(ct < limit_cmp)) continue;
+                const uint32_t ci = __shfl_sync(0xffffffffu, key_i, from), cp = __shfl_sync(0xffffffffu, key_p, from);
+                if (h.tri != 0xffffffffu && ct == h.t && !(ci < best_i || (ci == best_i && cp < best_p))) continue;
+                h.t = ct;
                 h.u = __shfl_sync(0xffffffffu, u, from);
                 h.v = __shfl_sync(0xffffffffu, v, from);
                 h.tri = __shfl_sync(0xffffffffu, tri, from);
                 h.front = __shfl_sync(0xffffffffu, front ? 1u : 0u, from);
-                limit_cmp = fminf(to, ray.tmax);
+                best_i = ci;
+                best_p = cp;
+                limit_cmp = next_up(ct);
+                if (!PARKED) admit = limit_cmp;
+            }
+            bound = limit_cmp;
+            if (settled < 32u && (hits >> settled) != 0u) {
+                float x = hit && lane >= settled && box_near <= t ? next_up(t) : INFINITY;
+                x = fminf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                x = fminf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    const float y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= uint32_t(o)) x = fminf(x, y);
+                }
+                x = __shfl_up_sync(0xffffffffu, x, 4);  // of the entries before this lane's
+                if (lane >= 4u) bound = fminf(bound, x);
             }
         }
-        // Entered children go back in place of what was taken.
-        const bool entered = near_t < limit_cmp;
-        const uint32_t mask = __ballot_sync(0xffffffffu, entered);
-        const float n1 = __shfl_xor_sync(0xffffffffu, near_t, 1), n2 = __shfl_xor_sync(0xffffffffu, near_t, 2),
-                    n3 = __shfl_xor_sync(0xffffffffu, near_t, 3);
-        if (entered) {
-            // Entered children of this node that are farther (equal: the later
-            // child), then those of nodes that were lower on the stack.
-            auto farther = [&](float n, uint32_t x) {
-                return n < limit_cmp && (n > near_t || (n == near_t && (child ^ x) > child)) ? 1u : 0u;
-            };
-            const uint32_t below = lane < 28u ? __popc(mask >> ((group + 1u) * 4u)) : 0u;
-            const uint32_t at = uint32_t(sp - take) + below + farther(n1, 1u) + farther(n2, 2u) + farther(n3, 3u);
-            stack[at] = make_uint2(child_entry, __float_as_uint(near_t));
+        // What stays goes back in place of what was taken: children, leaves with
+        // hits and, with PARKED, all that is not settled.
+        const bool entered = near_t < bound;
+        const uint32_t kids = __ballot_sync(0xffffffffu, entered) >> (group * 4u) & 15u;
+        const bool open = !ANY && lane >= settled && child == 0u && live && box_near < limit_cmp;
+        const bool mark = PARKED && open && lane > settled && count == 0u;
+        bool stays = entered;
+        if (open && kids == 0u && count != 0u) stays = PARKED || (hits >> lane & 15u) != 0u;
+        const uint32_t mask = __ballot_sync(0xffffffffu, stays);
+        const uint32_t marks = PARKED ? __ballot_sync(0xffffffffu, mark) : 0u;
+        // A node's children by wide_descend's network.
+        float n0 = __shfl_sync(0xffffffffu, near_t, int(lane & ~3u)), n1 = __shfl_sync(0xffffffffu, near_t, int(lane | 3u) - 2),
+              n2 = __shfl_sync(0xffffffffu, near_t, int(lane | 3u) - 1), n3 = __shfl_sync(0xffffffffu, near_t, int(lane | 3u));
+        uint32_t c0 = 0u, c1 = 1u, c2 = 2u, c3 = 3u;
+        order_pair(n0, c0, n1, c1);
+        order_pair(n2, c2, n3, c3);
+        order_pair(n0, c0, n2, c2);
+        order_pair(n1, c1, n3, c3);
+        order_pair(n1, c1, n2, c2);
+        uint32_t below = lane < 28u ? __popc(mask >> ((group + 1u) * 4u)) : 0u;
+        if (PARKED && lane < 28u) below += __popc(marks >> ((group + 1u) * 4u));
+        uint2* base = stack + (uint32_t(sp - take) + below);
+        if (stays) {
+            const uint32_t rank = c1 == child ? 1u : c2 == child ? 2u : c3 == child ? 3u : 0u;
+            base[entered ? __popc(kids) - 1u - rank : 0u] =
+                entered ? make_uint2(child_entry, __float_as_uint(near_t)) : e;
         }
-        sp += __popc(mask) - take;
+        if (mark) base[__popc(kids)] = make_uint2(kRefMask, e.y);
+        sp += __popc(mask) + __popc(marks) - take;
         __syncwarp();
     }
     return h;

@@ -171,10 +171,12 @@ __device__ __forceinline__ float4 intersect_one(const SceneSlot& sc, float4 o, f
 }
 
 // Queues up to this many rays per resident warp are traced a ray per warp
-// (trace_coop).  Swept in factors of two over whole frames: an 801x449 frame
-// went from 1,246 us to 1,110 at 2 and 1,097 at 4 and 8, a 256x256 Cornell
-// frame from 417 to 381 at 2 and 417 at 8, a 720p ReSTIR frame from 4,174 to
-// 4,086 at 2 and 4,183 at 8; a 1080p frame's tails are longer than that.
+// (trace_coop).  Swept in factors of two over whole frames, with a form that did
+// not keep the order of visits: an 801x449 frame went from 1,246 us to 1,110 at 2
+// and 1,097 at 4 and 8, a 256x256 Cornell frame from 417 to 381 at 2 and 417 at
+// 8, a 720p ReSTIR frame from 4,174 to 4,086 at 2 and 4,183 at 8; a 1080p frame's
+// tails are longer than that.  Keeping the order costs the first two (postponed
+// leaves) 3 % and 1.5 %, and the 1080p frame nothing.
 constexpr uint32_t kCoopRaysPerWarp = 2u;
 
 // 1024 threads per SM (at most 64 registers): traversal is issue-bound and
@@ -194,11 +196,11 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_intersect(WfDevice d, u
             if (coop) {
                 const float4 o = d.ray_o[q][w.base], dir = d.ray_d[q][w.base];
                 bool contested;
-                const TraceHit h = trace_coop<false>(d.scenes[d.ray_path[q][w.base] >> kPathBits].scene,
-                                                     TraceRay{from4(o), from4(dir), o.w, dir.w},
-                                                     TraceOptions{kInv, kInv, false}, stacks[threadIdx.x >> 5],
-                                                     contested);
-                // A contested hit is left to the loop below, on one lane.
+                const SceneSlot& sc = d.scenes[d.ray_path[q][w.base] >> kPathBits];
+                const TraceHit h = trace_coop<false, MODE == 2>(sc.scene, TraceRay{from4(o), from4(dir), o.w, dir.w},
+                                                                TraceOptions{kInv, kInv, false},
+                                                                stacks[threadIdx.x >> 5], contested);
+                // What is contested is left to the loop below, on one lane.
                 if (!contested) {
                     if (i < count) d.hit[i] = encode_hit(h);
                     i = count;

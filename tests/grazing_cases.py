@@ -88,7 +88,7 @@ def cells(seed, side, clutter):
         n = 20_000
         at = rng.integers(0, count, n)
         o = (home[at] + rng.uniform(-0.1, 0.1, (n, 3))).astype(F)
-        forward = rng.normal(size=(n, 3)).astype(F)
+        forward = unit(rng.normal(size=(n, 3)).astype(F))
         d = unit(forward)
         d64 = d.astype(np.float64)
         w = np.cross(d64, rng.normal(size=(n, 3)))

@@ -6,7 +6,11 @@ import pytest
 
 import grazing_cases as G
 from renderingengine_b200 import _native as N
+from renderingengine_b200 import scenes
+from renderingengine_b200.scenes import Camera
 from renderingengine_b200.traversal import Scene
+from renderingengine_b200.wavefront import (FILM_PRIMARY_IDENTITY, FILM_PRIMARY_POSITION, FILM_SAMPLE, Renderer,
+                                            frame_constants)
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +38,59 @@ def test_grazing_batches_equal_child_pair_loop(native, build, seed, side, clutte
             assert (want["metadata"][:, 1] == N.HIT_KIND_TRIANGLE).mean() > 0.9
             differ = (got.view(np.uint32).reshape(len(rays), -1) != want.view(np.uint32).reshape(len(rays), -1)).any(1)
             assert not differ.any(), f"{differ[:len(one)].sum()} of {len(one)} rays, any-hit {any_hit}"
+
+
+def _views(data, o, forward):
+    x = np.array([1.0, 0.0, 0.0], np.float32)
+    return [dict(frame=frame_constants(Camera(o[k], forward[k], x, x, 1e-30), 1, 1, 0, 4, seed=0x77 + k), offset=k,
+                 key=k) for k in range(len(o))]
+
+
+def _planes(scene, data, views, n, mode):
+    r = Renderer(1280, 832, 4)
+    r.set_scene(scene, data)
+    r.set_tuning(traversal=mode)
+    r.render_views(views)
+    assert r.collect().fatal_mask == 0
+    return [r.read_view(p, 0, n).view(np.uint32) for p in (FILM_PRIMARY_POSITION, FILM_PRIMARY_IDENTITY, FILM_SAMPLE)]
+
+
+SCENES = [(1, 4, 70), (2, 6, 30), (5, 6, 6), (6, 6, 150), (7, 6, 2)]
+
+
+@pytest.mark.parametrize("build", [N.BUILD_FLATTENED_SAH, N.BUILD_LBVH], ids=["sah", "lbvh"])
+@pytest.mark.parametrize("seed,side,clutter", SCENES)
+def test_grazing_short_queues_equal_long_ones(native, build, seed, side, clutter):
+    """Views of one pixel, each looking along a cell's ray, alone (a ray per
+    warp) and beside a view of a million pixels (32 rays per warp).  Mode 4 alone:
+    with postponed leaves (mode 2) the rays of a warp decide the order of visits
+    of one another."""
+    data, o, forward, _ = G.scene(seed, side, clutter)
+    scene = Scene(data.triangles, data.fingerprint, 1, build)
+    n = len(o)
+    views = _views(data, o, forward)
+    big = dict(frame=frame_constants(data.camera, 1280, 800, 0, 4, seed=0x51), offset=n, key=n)
+    alone, beside = _planes(scene, data, views, n, 4), _planes(scene, data, views + [big], n, 4)
+    assert len(np.unique(beside[1][:, 1])) > 0.9 * n  # every view sees its own cell
+    for a, b in zip(alone, beside):
+        assert not (a != b).any(), f"{(a != b).any(1).sum()} of {n} views"
+
+
+@pytest.mark.parametrize("mode", [2, 4])
+@pytest.mark.parametrize("build", [N.BUILD_FLATTENED_SAH, N.BUILD_LBVH], ids=["sah", "lbvh"])
+@pytest.mark.parametrize("seed,side,clutter", SCENES)
+def test_grazing_warp_per_ray_equals_lane_per_ray(native, build, seed, side, clutter, mode):
+    """A short queue gives each ray a warp, or one lane running the mode's loop
+    where the scene has alpha-masked triangles: here one that no ray meets."""
+    data, o, forward, _ = G.scene(seed, side, clutter)
+    far = scenes.canonical_triangles(np.array([[[50, 0, 0], [50, 1, 0], [50, 0, 1]]], np.float32), None, np.zeros(1, np.uint32),
+                                     np.full(1, len(data.triangles), np.uint32), np.zeros(1, np.uint32),
+                                     first_traversal_id=len(data.triangles))
+    data.triangles = np.concatenate([data.triangles, far])
+    planes = []
+    for masked in (False, True):
+        data.triangles["metadata"][-1, 0] |= 2 * masked  # RE_GEOMETRY_FLAG_ALPHA_MASK
+        scene = Scene(data.triangles, data.fingerprint, 1, build)
+        planes.append(_planes(scene, data, _views(data, o, forward), len(o), mode))
+    for a, b in zip(*planes):
+        assert not (a != b).any(), f"{(a != b).any(1).sum()} of {len(o)} views"
