@@ -919,7 +919,7 @@ re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth)
         return set_error(RE_RECORDING_FAILED, "four-wide layout exceeds its bound");
     uint32_t total = 0;
     for (uint32_t k = 0; k < level; ++k) total += host.count[k];
-    RE_CUDA_TRY(sc->wide_nodes.reserve(size_t(total) * sizeof(WideNode), true));
+    RE_CUDA_TRY(sc->wide_nodes.reserve(size_t(total) * sizeof(WideNode)));
     RE_CUDA_TRY(cudaMemcpyAsync(sc->wide_nodes.ptr, wide, size_t(total) * sizeof(WideNode), cudaMemcpyDeviceToDevice));
     sc->wide_node_count = total;
     sc->wide_stack_bound = host.stack_bound;
@@ -991,9 +991,9 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
     const auto t0 = std::chrono::steady_clock::now();
     // The passes read records as 16-byte lanes; records that start elsewhere
     // are moved first.
-    DeviceBuffer moved{true};
+    BuildBuffer moved;
     if ((reinterpret_cast<uintptr_t>(d_tris) & 15u) != 0u) {
-        RE_CUDA_TRY(moved.reserve(size_t(n) * sizeof(re_canonical_triangle), true));
+        RE_CUDA_TRY(moved.reserve(size_t(n) * sizeof(re_canonical_triangle)));
         RE_CUDA_TRY(cudaMemcpyAsync(moved.ptr, d_tris, size_t(n) * sizeof(re_canonical_triangle),
                                     cudaMemcpyDeviceToDevice));
         d_tris = static_cast<const re_canonical_triangle*>(moved.ptr);
@@ -1013,8 +1013,8 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
     const size_t o_keys_a = slot(size_t(n) * 8), o_keys_b = slot(size_t(n) * 8), o_vals_a = slot(size_t(n) * 4),
                  o_vals_b = slot(size_t(n) * 4), o_rows = slot(size_t(tiles) * kBins * 4), o_total = slot(kBins * 4),
                  o_box = slot(size_t(span) * 2 * sizeof(float4));
-    DeviceBuffer scratch{true};
-    RE_CUDA_TRY(scratch.reserve(std::max(bytes, o_reuse + wide_scratch_bytes(n)), true));
+    BuildBuffer scratch;
+    RE_CUDA_TRY(scratch.reserve(std::max(bytes, o_reuse + wide_scratch_bytes(n))));
     char* base = static_cast<char*>(scratch.ptr);
     auto* head = reinterpret_cast<BuildHeader*>(base + o_head);
     auto* seen = reinterpret_cast<uint32_t*>(base + o_seen);
@@ -1080,11 +1080,11 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
         }
     }
     RE_CUDA_TRY(cudaGetLastError());
-    RE_CUDA_TRY(sc->tris.reserve(size_t(n) * sizeof(DeviceTriangle), true));
-    RE_CUDA_TRY(sc->attrs.reserve(size_t(n) * sizeof(DeviceAttr), true));
-    RE_CUDA_TRY(sc->leaf_order.reserve(size_t(n) * 4, true));
+    RE_CUDA_TRY(sc->tris.reserve(size_t(n) * sizeof(DeviceTriangle)));
+    RE_CUDA_TRY(sc->attrs.reserve(size_t(n) * sizeof(DeviceAttr)));
+    RE_CUDA_TRY(sc->leaf_order.reserve(size_t(n) * 4));
     sc->alpha_masked = (hh.flags & kHasAlphaMask) != 0u;
-    if (sc->alpha_masked) RE_CUDA_TRY(sc->alpha_tc.reserve(size_t(n) * 2 * sizeof(float4), true));
+    if (sc->alpha_masked) RE_CUDA_TRY(sc->alpha_tc.reserve(size_t(n) * 2 * sizeof(float4)));
     const RangeBoxes boxes{reinterpret_cast<float4*>(base + o_box), span};
     k_pack_leaf_order<<<(n + 255) / 256, 256>>>(d_tris, vals_a, n, static_cast<DeviceTriangle*>(sc->tris.ptr),
                                                 static_cast<DeviceAttr*>(sc->attrs.ptr),
@@ -1105,7 +1105,7 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
     sc->flat.leaf_count = n;
     sc->flat_node_count = 2u * n - 1u;
     if (n > 1u) {
-        RE_CUDA_TRY(sc->nodes.reserve(size_t(n - 1u) * sizeof(DeviceNode), true));
+        RE_CUDA_TRY(sc->nodes.reserve(size_t(n - 1u) * sizeof(DeviceNode)));
         RE_CUDA_TRY(seg_build(boxes, n, nullptr));
         k_karras_nodes<<<(n - 1 + 255) / 256, 256>>>(keys_a, int(n), boxes, static_cast<DeviceNode*>(sc->nodes.ptr));
         RE_CUDA_TRY(cudaGetLastError());
@@ -1140,8 +1140,8 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
 // The same build from host records (validated by the caller).
 re_status build_lbvh_on_device(re_scene* sc, const re_canonical_triangle* tris) {
     const size_t bytes = size_t(sc->triangle_count) * sizeof(re_canonical_triangle);
-    DeviceBuffer records{true};
-    RE_CUDA_TRY(records.reserve(bytes, true));
+    BuildBuffer records;
+    RE_CUDA_TRY(records.reserve(bytes));
     RE_CUDA_TRY(cudaMemcpy(records.ptr, tris, bytes, cudaMemcpyHostToDevice));
     return build_lbvh_from_device_records(sc, static_cast<const re_canonical_triangle*>(records.ptr), false);
 }

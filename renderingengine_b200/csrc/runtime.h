@@ -43,21 +43,31 @@ static_assert(sizeof(DeviceAttr) == 64, "attribute record is 64 bytes");
 // Scratch buffer that grows on demand and is reused between calls.
 //
 // A pooled buffer comes from the device's scene pool (scene.cu) in place of
-// cudaMalloc.  It is ready on every stream when reserve returns and idle on
-// every stream before release gives it back, as with cudaMalloc and cudaFree,
-// except that an `ordered` one (a build's scratch and results until the build
-// synchronises) is only used on the legacy default stream meanwhile.
+// cudaMalloc.  It is ready on every stream when reserve returns, as with
+// cudaMalloc; unlike cudaFree, release does not wait: no work in flight may use
+// the buffer any more.
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
     bool pooled = false;
-    cudaError_t reserve(size_t n, bool ordered = false);
-    void release(bool ordered = false);
+    cudaError_t reserve(size_t n);
+    void release();
     DeviceBuffer() = default;
     explicit DeviceBuffer(bool from_pool) : pooled(from_pool) {}
     ~DeviceBuffer() { release(); }
 };
+
+// Pooled scratch of a build, used on the legacy default stream alone.
+struct BuildBuffer : DeviceBuffer {
+    BuildBuffer() : DeviceBuffer(true) {}
+    ~BuildBuffer() {
+        if (ptr != nullptr) cudaStreamSynchronize(cudaStreamLegacy);
+    }
+};
+
+// What the scene pool of `device` holds unused goes back to the device.
+void trim_scene_pool(int device);
 
 }  // namespace re
 
@@ -133,13 +143,13 @@ struct re_scene {
     // the persistent traversal kernels.
     re::DeviceBuffer stage_rays{true};
     re::DeviceBuffer stage_hits{true};
-    re::DeviceBuffer work_counter{true};
+    re::DeviceBuffer work_counter;
     // Quad nodes of trace batches, made with the first batch that walks them
     // (quad_state: 0 not asked for, 1 there, 2 no memory).
     re::DeviceBuffer quad_nodes{true};
     std::mutex quad_mutex;
     std::atomic<int> quad_state{0};
-    re::DeviceBuffer counters{true};
+    re::DeviceBuffer counters;
     // Four-wide nodes over the same triangles (re::WideNode): made with the
     // scene for this library's own trees, else on first use by a renderer
     // tuned for them.
@@ -148,20 +158,17 @@ struct re_scene {
     uint32_t wide_stack_bound = 0;
     // Eight-wide nodes, plain (re::Wide8Node) and compressed (re::Wide8QNode),
     // built on first use by a renderer tuned for them.
-    re::DeviceBuffer eight_nodes{true}, eight_qnodes{true};
+    re::DeviceBuffer eight_nodes, eight_qnodes;
     uint32_t eight_node_count = 0;
     uint32_t eight_stack_bound = 0;
     // Alpha masks: per leaf-ordered triangle texture coordinates + material
     // (2 x float4, made when any triangle is alpha-masked), and the tables
     // of re_scene_set_alpha_masks with their device AlphaView.
     bool alpha_masked = false;
-    re::DeviceBuffer alpha_tc{true}, alpha_materials{true}, alpha_atlas{true}, alpha_view{true};
+    re::DeviceBuffer alpha_tc, alpha_materials, alpha_atlas, alpha_view;
     // Copy streams of chunked host-memory trace batches (created on first use).
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
-    ~re_scene() {
-        if (copy_in) cudaStreamDestroy(copy_in);
-        if (copy_out) cudaStreamDestroy(copy_out);
-    }
+    ~re_scene();  // waits for the device's work in flight, as cudaFree does
 };
 
 namespace re {

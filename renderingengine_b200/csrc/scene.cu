@@ -30,66 +30,89 @@ namespace {
 // Memory of scenes and of their builds.  A cudaMalloc takes about 350 us here
 // and a cudaFree 300, whatever the size, and a scene holds half a dozen
 // buffers: a 606,208-triangle rebuild from device records spent 4 of its 5 ms
-// in them.  The pool keeps at most this much of what is freed, and gives it
-// back when an allocation of the library fails.
+// in them.  The pool keeps at most this much of what is freed; the driver takes
+// it back for any allocation of the process that needs it.
 constexpr uint64_t kScenePoolKeeps = 256ull << 20;
 
+// The pool allocates and frees on a stream of its own that does nothing else and
+// does not wait for the legacy default stream, so neither is refused, or ends a
+// capture, while another thread captures a stream.  The small allocation keeps a
+// block of the driver's small allocations open: beside it, a scene's work counter
+// takes 1 us to allocate and 3 to free.
+struct ScenePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    void* small = nullptr;
+};
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pools[64] = {};
+ScenePool g_pools[64];
 
-cudaError_t scene_pool(int device, cudaMemPool_t* out) {
+cudaError_t scene_pool(int device, ScenePool* out) {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (g_pools[device] == nullptr) {
+    ScenePool& p = g_pools[device];
+    if (p.pool == nullptr) {
+        ScenePool made;
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        cudaError_t e = cudaMemPoolCreate(&pool, &props);
-        if (e != cudaSuccess) return e;
         uint64_t keep = kScenePoolKeeps;
-        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        cudaError_t e = cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaMemPoolCreate(&made.pool, &props);
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e == cudaSuccess) e = cudaMalloc(&made.small, 4);
         if (e != cudaSuccess) {
-            cudaMemPoolDestroy(pool);
+            if (made.pool != nullptr) cudaMemPoolDestroy(made.pool);
+            if (made.stream != nullptr) cudaStreamDestroy(made.stream);
             return e;
         }
-        g_pools[device] = pool;
+        p = made;
     }
-    *out = g_pools[device];
+    *out = p;
     return cudaSuccess;
 }
 
-// What the pool holds unused goes back to the device.
-void trim_scene_pool(int device) {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (device < 0 || device >= 64 || g_pools[device] == nullptr) return;
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(g_pools[device], 0);
-}
-
-cudaError_t raw_allocate(void** ptr, size_t n, bool pooled, int device) {
-    if (!pooled) return cudaMalloc(ptr, n);
-    cudaMemPool_t pool = nullptr;
-    const cudaError_t e = scene_pool(device, &pool);
-    return e != cudaSuccess ? e : cudaMallocFromPoolAsync(ptr, n, pool, cudaStreamLegacy);
-}
+// Makes a device current for a scope.
+struct DeviceScope {
+    int before = 0, device;
+    explicit DeviceScope(int d) : device(d) {
+        cudaGetDevice(&before);
+        if (before != device) cudaSetDevice(device);
+    }
+    ~DeviceScope() {
+        if (before != device) cudaSetDevice(before);
+    }
+};
 
 }  // namespace
 
-cudaError_t DeviceBuffer::reserve(size_t n, bool ordered) {
+void trim_scene_pool(int device) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (device < 0 || device >= 64 || g_pools[device].pool == nullptr) return;
+    cudaStreamSynchronize(g_pools[device].stream);
+    cudaMemPoolTrimTo(g_pools[device].pool, 0);
+}
+
+cudaError_t DeviceBuffer::reserve(size_t n) {
     if (n <= bytes && ptr != nullptr) return cudaSuccess;
-    release(ordered);
+    release();
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     const size_t want = n == 0 ? 16 : n;
-    e = raw_allocate(&ptr, want, pooled, device);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        trim_scene_pool(device);
-        e = raw_allocate(&ptr, want, pooled, device);
+    if (!pooled) {
+        e = cudaMalloc(&ptr, want);
+    } else {
+        ScenePool p;
+        e = scene_pool(device, &p);
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ptr, want, p.pool, p.stream);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            trim_scene_pool(device);
+            e = cudaMallocFromPoolAsync(&ptr, want, p.pool, p.stream);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(p.stream);
     }
-    if (e == cudaSuccess && pooled && !ordered) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
         ptr = nullptr;
         bytes = 0;
@@ -99,18 +122,12 @@ cudaError_t DeviceBuffer::reserve(size_t n, bool ordered) {
     return cudaSuccess;
 }
 
-void DeviceBuffer::release(bool ordered) {
+void DeviceBuffer::release() {
     if (ptr != nullptr) {
-        int cur = 0;
-        cudaGetDevice(&cur);
-        if (cur != device) cudaSetDevice(device);
-        if (!pooled) {
-            cudaFree(ptr);
-        } else {
-            if (!ordered) cudaDeviceSynchronize();
-            cudaFreeAsync(ptr, cudaStreamLegacy);
-        }
-        if (cur != device) cudaSetDevice(cur);
+        DeviceScope on(device);
+        ScenePool p;
+        if (!pooled) cudaFree(ptr);
+        else if (scene_pool(device, &p) == cudaSuccess) cudaFreeAsync(ptr, p.stream);
     }
     ptr = nullptr;
     bytes = 0;
@@ -457,8 +474,8 @@ re_status run_trace_chunked(re_scene* sc, const re_trace_batch* b, cudaStream_t 
         ok(cudaMemcpyAsync(b->hits + b->hit_offset + off, d_hits + off, size_t(cnt) * sizeof(re_hit_record),
                            cudaMemcpyDeviceToHost, sc->copy_out));
     }
-    ok(cudaStreamSynchronize(sc->copy_out));
-    ok(cudaStreamSynchronize(stream));
+    // Also after an error: the staging buffers are idle when the call returns.
+    for (cudaStream_t s : {sc->copy_in, sc->copy_out, stream}) ok(cudaStreamSynchronize(s));
     for (uint32_t k = 0; k < chunks; ++k) {
         if (in[k]) cudaEventDestroy(in[k]);
         if (run[k]) cudaEventDestroy(run[k]);
@@ -479,6 +496,14 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
     const re_ray_record* d_rays = b->rays + b->ray_offset;
     re_hit_record* d_hits = b->hits + b->hit_offset;
     const bool host = b->memory == RE_MEMORY_HOST;
+    // The staging buffers are idle when a call returns, also by an error.
+    struct Idle {
+        cudaStream_t stream;
+        bool pending;
+        ~Idle() {
+            if (pending) cudaStreamSynchronize(stream);
+        }
+    } idle{stream, host};
     if (host) {
         RE_CUDA_TRY(sc->stage_rays.reserve(ray_bytes));
         RE_CUDA_TRY(sc->stage_hits.reserve(hit_bytes));
@@ -524,6 +549,7 @@ re_status run_trace(re_scene* sc, const re_trace_batch* b, bool any, re_traversa
     }
     if (host) {
         RE_CUDA_TRY(cudaMemcpyAsync(b->hits + b->hit_offset, d_hits, hit_bytes, cudaMemcpyDeviceToHost, stream));
+        idle.pending = false;
         RE_CUDA_TRY(cudaStreamSynchronize(stream));
     }
     return clear_error();
@@ -565,10 +591,11 @@ void reserve_work_counter(re_scene* sc) {
 // the scene stands and traces over its child pairs.
 void make_wide_nodes(re_scene* sc) {
     if (sc->layout_meta.root_is_leaf != 0u) return;
-    DeviceBuffer scratch{true};
+    BuildBuffer scratch;
     if (scratch.reserve(wide_scratch_bytes(sc->device_node_count)) != cudaSuccess ||
         build_wide_on_device(sc, scratch.ptr, nullptr) != RE_SUCCESS) {
         cudaGetLastError();
+        cudaStreamSynchronize(cudaStreamLegacy);
         sc->wide_nodes.release();
         sc->wide_node_count = sc->wide_stack_bound = 0u;
     }
@@ -643,6 +670,18 @@ re_status upload_scene_triangles(re_scene* sc, const re_canonical_triangle* src_
 }  // namespace re
 
 using namespace re;
+
+// The pooled members go back to the pool without a wait, so what may still read
+// them, the caller's graphs among it, is waited for here: by cudaFree, which is
+// open beside a thread-local or relaxed stream capture, where a device-wide
+// synchronise is refused and ends the capture.
+re_scene::~re_scene() {
+    DeviceScope on(device);
+    if (copy_in) cudaStreamDestroy(copy_in);
+    if (copy_out) cudaStreamDestroy(copy_out);
+    if (work_counter.ptr != nullptr) work_counter.release();
+    else cudaDeviceSynchronize();
+}
 
 extern "C" {
 

@@ -1,0 +1,98 @@
+"""Scene memory beside the caller's own work: captures of other streams, work
+in flight, and what a scene reports to hold."""
+import threading
+
+import numpy as np
+import pytest
+
+from renderingengine_b200 import _native as N
+from renderingengine_b200 import scenes
+from renderingengine_b200.traversal import Scene
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(build=N.BUILD_LBVH, triangles=20_000):
+    return Scene(scenes.triangle_soup(triangles, seed=9).triangles, 5, 1, build)
+
+
+def _rays(count, seed=1):
+    rng = np.random.default_rng(seed)
+    r = np.zeros(count, N.RAY_DTYPE)
+    d = rng.normal(size=(count, 3))
+    r["origin_tmin"][:, :3], r["origin_tmin"][:, 3] = rng.random((count, 3)), 1e-4
+    r["direction_tmax"][:, :3], r["direction_tmax"][:, 3] = d / np.linalg.norm(d, axis=1, keepdims=True), 1e30
+    return r
+
+
+def _beside_capture(mode, call):
+    """`call` in another thread (mode thread_local) or this one (relaxed) while
+    this thread captures; the capture must end and replay."""
+    import torch
+    x = torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    errors = []
+
+    def run():
+        try:
+            torch.cuda.set_device(0)
+            call()
+        except Exception as e:  # reported by the caller's thread
+            errors.append(e)
+
+    with torch.cuda.graph(graph, capture_error_mode=mode):
+        x.add_(1.0)
+        if mode == "thread_local":
+            t = threading.Thread(target=run)
+            t.start()
+            t.join()
+        else:
+            run()
+    assert not errors, errors
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1000.0
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+@pytest.mark.parametrize("build", [N.BUILD_LBVH, N.BUILD_FLATTENED_SAH], ids=["lbvh", "sah"])
+def test_scene_destroyed_beside_a_capture(native, mode, build):
+    scene = _scene(build)
+    scene.trace(_rays(300_000), any_hit=True)
+    _beside_capture(mode, scene.close)
+
+
+def test_host_batch_that_grows_its_staging_beside_a_capture(native):
+    scene = _scene()
+    rays = _rays(5000)
+    scene.trace(rays[:100])
+    want, _ = scene.trace(rays, counters=True)
+    fresh = _scene()
+    fresh.trace(rays[:100])
+    got = []
+    _beside_capture("thread_local", lambda: got.append(fresh.trace(rays)))
+    np.testing.assert_array_equal(got[0].view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("build", [N.BUILD_LBVH, N.BUILD_FLATTENED_SAH], ids=["lbvh", "sah"])
+def test_scene_destroyed_with_work_in_flight(native, build):
+    """Destroying waits for what may still read the scene, on any stream."""
+    import torch
+    scene = _scene(build)
+    rays = _rays(50_000)
+    want, _ = scene.trace(rays, counters=True)
+    d_rays = torch.from_numpy(rays.view(np.uint8).reshape(-1)).cuda()
+    d_hits = torch.zeros(len(rays) * N.HIT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    stream, done = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)  # about 10 ms
+        scene.trace_device(d_rays.data_ptr(), d_hits.data_ptr(), len(rays), stream=stream.cuda_stream)
+        done.record()
+    scene.close()
+    assert done.query()
+    other = _scene(build, 30_000)  # takes the memory that was given back
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(d_hits.cpu().numpy().view(np.uint32), want.view(np.uint32).reshape(-1))
+    other.close()
