@@ -866,7 +866,8 @@ RE_API re_status re_scene_info_get(const re_scene* sc, re_scene_info* out) {
     out->max_depth = sc->flat.max_depth;
     out->leaf_count = sc->flat.leaf_count;
     out->device_bytes = uint64_t(sc->nodes.bytes) + sc->tris.bytes + sc->attrs.bytes +
-                        sc->leaf_order.bytes + sc->wide_nodes.bytes;
+                        sc->leaf_order.bytes + sc->wide_nodes.bytes +
+                        (sc->quad_state.load(std::memory_order_acquire) == 1 ? sc->quad_nodes.bytes : 0u);
     out->build_ms = sc->build_ms;
     out->node_bytes = sizeof(DeviceNode);
     out->triangle_bytes = sizeof(DeviceTriangle);

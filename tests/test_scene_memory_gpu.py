@@ -96,3 +96,12 @@ def test_scene_destroyed_with_work_in_flight(native, build):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(d_hits.cpu().numpy().view(np.uint32), want.view(np.uint32).reshape(-1))
     other.close()
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_device_bytes_count_the_quad_nodes(native, any_hit):
+    triangles = 20_000
+    scene = _scene(N.BUILD_LBVH, triangles)
+    before = scene.info().device_bytes
+    scene.trace(_rays(1 << 18), any_hit=any_hit)
+    assert scene.info().device_bytes == before + 128 * (triangles - 1)  # one for each pair of children
