@@ -970,16 +970,22 @@ __global__ void k_quad_nodes(const DeviceNode* nodes, uint32_t count, WideNode* 
 
 }  // namespace
 
-// Makes the scene's quad nodes; false when it has no memory for them.
 bool make_quad_nodes(re_scene* sc, cudaStream_t stream) {
-    if (sc->quad_nodes.reserve(size_t(sc->device_node_count) * sizeof(WideNode)) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+    const uint32_t n = sc->device_node_count;
+    bool ok = sc->quad_event != nullptr ||
+              cudaEventCreateWithFlags(&sc->quad_event, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && sc->quad_nodes.reserve_on(size_t(n) * sizeof(WideNode), stream) == cudaSuccess;
+    if (ok) {
+        k_quad_nodes<<<(n + 127u) / 128u, 128, 0, stream>>>(static_cast<const DeviceNode*>(sc->nodes.ptr), n,
+                                                            static_cast<WideNode*>(sc->quad_nodes.ptr));
+        ok = cudaGetLastError() == cudaSuccess && cudaEventRecord(sc->quad_event, stream) == cudaSuccess;
+        if (!ok) {
+            cudaStreamSynchronize(stream);
+            sc->quad_nodes.release();
+        }
     }
-    k_quad_nodes<<<(sc->device_node_count + 127u) / 128u, 128, 0, stream>>>(
-        static_cast<const DeviceNode*>(sc->nodes.ptr), sc->device_node_count,
-        static_cast<WideNode*>(sc->quad_nodes.ptr));
-    return cudaStreamSynchronize(stream) == cudaSuccess;  // later batches may use any stream
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 // The scene from CanonicalTraversalTriangle records in device memory: the

@@ -52,6 +52,9 @@ struct DeviceBuffer {
     int device = 0;
     bool pooled = false;
     cudaError_t reserve(size_t n);
+    // Pooled and empty only: ready on `stream` alone, in its order, without a
+    // wait or a retry.
+    cudaError_t reserve_on(size_t n, cudaStream_t stream);
     void release();
     DeviceBuffer() = default;
     explicit DeviceBuffer(bool from_pool) : pooled(from_pool) {}
@@ -87,7 +90,8 @@ re_status build_lbvh_from_device_records(re_scene* sc, const re_canonical_triang
 // `scratch` (wide_scratch_bytes of the child-pair node count).
 size_t wide_scratch_bytes(uint32_t interior);
 re_status build_wide_on_device(re_scene* sc, void* scratch, uint32_t* max_depth);
-// Quad nodes of the scene's child pairs (traverse.cuh, trace_quad).
+// Queues making the quad nodes of the scene's child pairs (traverse.cuh,
+// trace_quad) on `stream`; false, with nothing left behind, when that fails.
 bool make_quad_nodes(re_scene* sc, cudaStream_t stream);
 // Fills sc->flat's nodes and leaf order when the tree was built on the device.
 re_status host_flat(const re_scene* sc);
@@ -144,11 +148,14 @@ struct re_scene {
     re::DeviceBuffer stage_rays{true};
     re::DeviceBuffer stage_hits{true};
     re::DeviceBuffer work_counter;
-    // Quad nodes of trace batches, made with the first batch that walks them
-    // (quad_state: 0 not asked for, 1 there, 2 no memory).
+    // Quad nodes of trace batches, made on the stream of the batch that is the
+    // first to walk them.
+    enum QuadState { kQuadNone, kQuadQueued, kQuadReady };  // queued: there behind quad_event
     re::DeviceBuffer quad_nodes{true};
+    cudaEvent_t quad_event = nullptr;
     std::mutex quad_mutex;
-    std::atomic<int> quad_state{0};
+    std::atomic<int> quad_state{kQuadNone};
+    std::atomic<uint64_t> quad_owed{0};  // rays of batches without them since the last attempt
     re::DeviceBuffer counters;
     // Four-wide nodes over the same triangles (re::WideNode): made with the
     // scene for this library's own trees, else on first use by a renderer

@@ -122,6 +122,16 @@ cudaError_t DeviceBuffer::reserve(size_t n) {
     return cudaSuccess;
 }
 
+cudaError_t DeviceBuffer::reserve_on(size_t n, cudaStream_t stream) {
+    ScenePool p;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = scene_pool(device, &p);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ptr, n, p.pool, stream);
+    if (e == cudaSuccess) bytes = n;
+    else ptr = nullptr;
+    return e;
+}
+
 void DeviceBuffer::release() {
     if (ptr != nullptr) {
         DeviceScope on(device);
@@ -362,36 +372,63 @@ cudaError_t launch_batch_k(re_scene* sc, const BatchArgs& args, cudaStream_t str
 
 // Batches over the quad nodes: on the library's own trees (in a caller's
 // flattened nodes a child's box need not be the union of its children's), where
-// the scene has quad nodes.  They are made, once, by the first batch (not being
-// captured) that by itself gains what they cost, a pass over the nodes of about
-// 30 us for 606,208 triangles and a few launches' time.  Random rays, quad nodes
-// / child pairs: 262,144 any-hit rays, soups of 1,000 triangles 101 / 117 us,
-// 16,000 274 / 337, 60,000 383 / 477, the 606,208 145 / 171 (camera rays 182 /
-// 254); closest hits 112 / 124, 297 / 355, 422 / 509, 167 / 191 (camera rays
-// 224 / 270).  With the nodes there 500 any-hit rays take 19 / 23, 39 / 50,
-// 64 / 80 and 33 / 46, closest 21 / 23, 41 / 52, 66 / 82 and 35 / 47.  Over the
-// 36 triangles of a Cornell box they are equal.
-constexpr uint32_t kQuadMakingRays = 1u << 18;
+// the scene has quad nodes.  They are made, on its stream, by a batch (not being
+// captured) once the batches without them have had as many rays as would gain what
+// they cost, a pass over the nodes of about 30 us for 606,208 triangles and a few
+// launches' time; a batch too small to fill the device gains as a larger one.
+// Random rays, quad nodes / child pairs: 262,144 any-hit rays, soups of 1,000
+// triangles 101 / 117 us, 16,000 274 / 337, 60,000 383 / 477, the 606,208 145 /
+// 171 (camera rays 182 / 254); closest hits 112 / 124, 297 / 355, 422 / 509, 167 /
+// 191 (camera rays 224 / 270).  With the nodes there 500 any-hit rays take 19 /
+// 23, 39 / 50, 64 / 80 and 33 / 46, closest 21 / 23, 41 / 52, 66 / 82 and 35 / 47.
+// Over the 36 triangles of a Cornell box they are equal.
+//
+// The call stays asynchronous: nothing waits here, other streams wait on the device.
+// An attempt that fails is repeated when as many rays have been traced again.
+constexpr uint32_t kQuadMakingRays = 1u << 18, kQuadLeastRays = 1u << 14;
 const float4* quad_nodes(re_scene* sc, uint32_t count, cudaStream_t stream) {
     if (!sc->own_tree || sc->layout_meta.root_is_leaf != 0u || sc->flat.max_depth > 64u) return nullptr;
-    if (sc->quad_state.load(std::memory_order_acquire) == 0 && count >= kQuadMakingRays &&
-        count >= sc->triangle_count / 2u) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return nullptr;
-        }
+    const auto ready = [sc] { return static_cast<const float4*>(sc->quad_nodes.ptr); };
+    int state = sc->quad_state.load(std::memory_order_acquire);
+    if (state == re_scene::kQuadReady) return ready();
+    const uint64_t cost = std::max(kQuadMakingRays, sc->triangle_count);
+    if (state == re_scene::kQuadNone) {
+        const uint64_t rays = std::max(kQuadLeastRays, count);
+        if (sc->quad_owed.fetch_add(rays, std::memory_order_relaxed) + rays < cost) return nullptr;
+    }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    // Another thread may be capturing a stream of its own.
+    struct Relaxed {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    } relaxed;
+    if (state == re_scene::kQuadNone) {
         std::lock_guard<std::mutex> lock(sc->quad_mutex);
-        if (sc->quad_state.load(std::memory_order_relaxed) == 0) {
-            // Another thread may be capturing a stream of its own.
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            sc->quad_state.store(make_quad_nodes(sc, stream) ? 1 : 2, std::memory_order_release);
-            cudaThreadExchangeStreamCaptureMode(&mode);
+        state = sc->quad_state.load(std::memory_order_relaxed);
+        if (state == re_scene::kQuadNone) {
+            sc->quad_owed.store(0, std::memory_order_relaxed);
+            if (!make_quad_nodes(sc, stream)) return nullptr;
+            sc->quad_state.store(re_scene::kQuadQueued, std::memory_order_release);
+            return ready();
         }
     }
-    return sc->quad_state.load(std::memory_order_acquire) == 1 ? static_cast<const float4*>(sc->quad_nodes.ptr)
-                                                               : nullptr;
+    if (state == re_scene::kQuadQueued) {
+        if (cudaEventQuery(sc->quad_event) == cudaSuccess) {
+            sc->quad_state.store(re_scene::kQuadReady, std::memory_order_release);
+        } else {
+            cudaGetLastError();
+            if (cudaStreamWaitEvent(stream, sc->quad_event, 0) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+        }
+    }
+    return ready();
 }
 
 template <bool ANY, bool COUNT>
@@ -679,6 +716,7 @@ re_scene::~re_scene() {
     DeviceScope on(device);
     if (copy_in) cudaStreamDestroy(copy_in);
     if (copy_out) cudaStreamDestroy(copy_out);
+    if (quad_event) cudaEventDestroy(quad_event);
     if (work_counter.ptr != nullptr) work_counter.release();
     else cudaDeviceSynchronize();
 }
@@ -867,7 +905,7 @@ RE_API re_status re_scene_info_get(const re_scene* sc, re_scene_info* out) {
     out->leaf_count = sc->flat.leaf_count;
     out->device_bytes = uint64_t(sc->nodes.bytes) + sc->tris.bytes + sc->attrs.bytes +
                         sc->leaf_order.bytes + sc->wide_nodes.bytes +
-                        (sc->quad_state.load(std::memory_order_acquire) == 1 ? sc->quad_nodes.bytes : 0u);
+                        (sc->quad_state.load(std::memory_order_acquire) != re_scene::kQuadNone ? sc->quad_nodes.bytes : 0u);
     out->build_ms = sc->build_ms;
     out->node_bytes = sizeof(DeviceNode);
     out->triangle_bytes = sizeof(DeviceTriangle);

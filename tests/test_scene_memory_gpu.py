@@ -105,3 +105,66 @@ def test_device_bytes_count_the_quad_nodes(native, any_hit):
     before = scene.info().device_bytes
     scene.trace(_rays(1 << 18), any_hit=any_hit)
     assert scene.info().device_bytes == before + 128 * (triangles - 1)  # one for each pair of children
+
+
+def _device(rays):
+    import torch
+    return (torch.from_numpy(rays.view(np.uint8).reshape(-1)).cuda(),
+            torch.zeros(len(rays) * N.HIT_DTYPE.itemsize, dtype=torch.uint8, device="cuda"))
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("busy", ["own", "default"])
+def test_device_batches_do_not_wait(native, any_hit, busy):
+    """A scene's first large batch, with its stream or the default stream busy,
+    returns before either is done; the next one, on another stream, has the same
+    hits."""
+    import torch
+    scene = _scene()
+    rays = _rays(1 << 18)
+    want, _ = scene.trace(rays, any_hit=any_hit, counters=True)
+    scene.close()
+    scene = _scene()
+    batches = [_device(rays), _device(rays)]
+    torch.cuda.synchronize()
+    first, second, done = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(first if busy == "own" else torch.cuda.default_stream()):
+        torch.cuda._sleep(400_000_000)  # about 200 ms
+        done.record()
+    for stream, (d_rays, d_hits) in zip((first, second), batches):
+        second.wait_stream(first)  # a scene's batches share its work counter
+        scene.trace_device(d_rays.data_ptr(), d_hits.data_ptr(), len(rays), any_hit, stream=stream.cuda_stream)
+    assert not done.query()
+    torch.cuda.synchronize()
+    for _, d_hits in batches:
+        np.testing.assert_array_equal(d_hits.cpu().numpy().view(np.uint32), want.view(np.uint32).reshape(-1))
+    scene.close()
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_quad_nodes_made_beside_a_capture_of_a_blocking_stream(native, any_hit):
+    """Beside such a capture the legacy default stream is closed.  The batch gets
+    its quad nodes all the same, and the capture its end."""
+    import ctypes
+
+    import torch
+    scene = _scene()
+    before = scene.info().device_bytes
+    rays = _rays(1 << 18)
+    want, _ = scene.trace(rays[:1000], any_hit=any_hit, counters=True)
+    d_rays, d_hits = _device(rays)
+    x = torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    handle = ctypes.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0  # blocking, unlike torch's
+    own = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(handle.value), capture_error_mode="relaxed"):
+        x.add_(1.0)
+        scene.trace_device(d_rays.data_ptr(), d_hits.data_ptr(), len(rays), any_hit, stream=own.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1000.0
+    assert scene.info().device_bytes > before
+    got = d_hits.cpu().numpy().view(N.HIT_DTYPE)[:1000]
+    np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
