@@ -14,6 +14,7 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <string>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -37,7 +38,7 @@ struct SceneRecord {
     float radius = 1.0f;
     re_scene* scene = nullptr;  // resident build, or null
     int slot = -1;
-    uint64_t bytes = 0;
+    uint64_t bytes = 0;  // scene_bytes of its last build
 };
 
 // A step takes further samples of its requests up to this many paths in all:
@@ -57,23 +58,25 @@ struct Request {
     size_t result_bytes = 0;
 };
 
-// Device bytes a resident scene is charged: child-pair nodes, triangles and
-// attributes plus the renderer's per-slot tables.  (The four-wide nodes and the
-// build's leaf order have never been part of the charge.)
+// Device bytes a resident scene takes: all that the scene holds
+// (re_scene_info.device_bytes) plus the renderer's per-slot tables.
 uint64_t scene_bytes(const SceneRecord& rec, const re_scene_info& info) {
-    return info.device_bytes - rec.scene->wide_nodes.bytes - rec.scene->leaf_order.bytes + uint64_t(rec.tris.size()) * 4u +
-           rec.materials.size() * sizeof(re_material) + rec.lights.size() * (sizeof(re_light) + 24u) +
-           rec.fixtures.size() * sizeof(re_float4);
+    return info.device_bytes + uint64_t(rec.tris.size()) * 4u + rec.materials.size() * sizeof(re_material) +
+           rec.lights.size() * (sizeof(re_light) + 24u) + rec.fixtures.size() * sizeof(re_float4);
 }
 
-// Charge of a scene before it is built: an upper bound of scene_bytes (a
-// binary hierarchy has at most two nodes per triangle) plus 1 MiB for the
-// builder's transient scratch.
+// What must be free of the budget before a scene is built.  Per triangle 196
+// bytes of child pairs, triangles, attributes and slot table, and 64 and 1 MiB
+// for the leaf order and the four-wide nodes: those take 40 to 55 bytes of a usual
+// tree and 85 of a perfectly regular one, so scene_bytes is compared again when
+// they are there, and a scene built before is known.  The build's scratch, given
+// back before make_resident returns, is not part of it.
 uint64_t scene_charge(const SceneRecord& rec) {
     const uint64_t n = rec.tris.size();
-    return n * (2u * sizeof(re::DeviceNode) + sizeof(re::DeviceTriangle) + sizeof(re::DeviceAttr) + 4u) +
-           rec.materials.size() * sizeof(re_material) + rec.lights.size() * (sizeof(re_light) + 24u) +
-           rec.fixtures.size() * sizeof(re_float4) + (1u << 20);
+    return std::max(rec.bytes,
+                    n * (2u * sizeof(re::DeviceNode) + sizeof(re::DeviceTriangle) + sizeof(re::DeviceAttr) + 4u) +
+                        rec.materials.size() * sizeof(re_material) + rec.lights.size() * (sizeof(re_light) + 24u) +
+                        rec.fixtures.size() * sizeof(re_float4) + (1u << 20));
 }
 
 }  // namespace
@@ -155,16 +158,21 @@ void evict(re_server* s, uint64_t key) {
 re_status make_resident(re_server* s, uint64_t key, bool may_evict = true) {
     SceneRecord& rec = s->scenes.at(key);
     if (rec.scene != nullptr) return RE_SUCCESS;
-    const uint64_t estimate = scene_charge(rec);
     const uint64_t budget = s->desc.hbm_budget_bytes;
-    if (s->fixed_bytes + estimate > budget)
-        return set_error(RE_BUDGET_EXCEEDED, "scene does not fit the HBM budget");
-    if (s->fixed_bytes + s->lru.bytes() + estimate > budget) {
-        if (!may_evict) return set_error(RE_BUDGET_EXCEEDED, "scene does not fit beside the resident ones");
-        const auto vict = s->lru.victims(budget - s->fixed_bytes - estimate);
-        if (vict.empty()) return set_error(RE_BUDGET_EXCEEDED, "no evictable scene frees enough of the budget");
-        for (uint64_t v : vict) evict(s, v);
-    }
+    // Room for `bytes` beside the path pool and the resident scenes.
+    auto make_room = [&](uint64_t bytes) {
+        if (s->fixed_bytes + bytes > budget)
+            return set_error(RE_BUDGET_EXCEEDED, "scene does not fit the HBM budget");
+        if (s->fixed_bytes + s->lru.bytes() + bytes > budget) {
+            if (!may_evict) return set_error(RE_BUDGET_EXCEEDED, "scene does not fit beside the resident ones");
+            const auto vict = s->lru.victims(budget - s->fixed_bytes - bytes);
+            if (vict.empty()) return set_error(RE_BUDGET_EXCEEDED, "no evictable scene frees enough of the budget");
+            for (uint64_t v : vict) evict(s, v);
+        }
+        return RE_SUCCESS;
+    };
+    re_status st = make_room(scene_charge(rec));
+    if (st != RE_SUCCESS) return st;
     int slot = -1;
     for (int k = 0; k < int(RE_MAX_SCENE_SLOTS); ++k)
         if (!s->slot_used[k]) {
@@ -191,20 +199,26 @@ re_status make_resident(re_server* s, uint64_t key, bool may_evict = true) {
     d.fingerprint = key + 1u;
     d.generation = 1;
     d.device = s->desc.device;
-    re_status st = re_scene_create(&d, &rec.scene);
+    st = re_scene_create(&d, &rec.scene);
     if (st != RE_SUCCESS) return st;
-    st = re_renderer_bind_scene(s->renderer, uint32_t(slot), rec.scene, rec.materials.data(),
-                                uint32_t(rec.materials.size()), rec.lights.empty() ? nullptr : rec.lights.data(),
-                                uint32_t(rec.lights.size()), rec.fixtures.empty() ? nullptr : rec.fixtures.data(),
-                                uint32_t(rec.fixtures.size() / 4), rec.light_selection, rec.radius);
-    if (st != RE_SUCCESS) {
-        re_scene_destroy(rec.scene);
-        rec.scene = nullptr;
-        return st;
-    }
     re_scene_info info{};
     re_scene_info_get(rec.scene, &info);
     rec.bytes = scene_bytes(rec, info);
+    st = make_room(rec.bytes);
+    // The pool's unused memory, scratch and evicted scenes, is no one's charge.
+    trim_scene_pool(int(s->desc.device));
+    if (st == RE_SUCCESS)
+        st = re_renderer_bind_scene(s->renderer, uint32_t(slot), rec.scene, rec.materials.data(),
+                                    uint32_t(rec.materials.size()), rec.lights.empty() ? nullptr : rec.lights.data(),
+                                    uint32_t(rec.lights.size()), rec.fixtures.empty() ? nullptr : rec.fixtures.data(),
+                                    uint32_t(rec.fixtures.size() / 4), rec.light_selection, rec.radius);
+    if (st != RE_SUCCESS) {
+        const std::string why = re_last_error();
+        re_scene_destroy(rec.scene);
+        trim_scene_pool(int(s->desc.device));
+        rec.scene = nullptr;
+        return set_error(st, why);
+    }
     rec.slot = slot;
     s->slot_used[slot] = true;
     s->lru.insert(key, rec.bytes, ++s->stamp);
