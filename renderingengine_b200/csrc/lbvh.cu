@@ -1162,9 +1162,17 @@ re_status host_flat(const re_scene* csc) {
     const uint32_t n = sc->triangle_count;
     std::vector<DeviceNode> dev(n - 1u);
     std::vector<uint32_t> order(n);
-    RE_CUDA_TRY(cudaSetDevice(sc->device));
-    RE_CUDA_TRY(cudaMemcpy(dev.data(), sc->nodes.ptr, dev.size() * sizeof(DeviceNode), cudaMemcpyDeviceToHost));
-    RE_CUDA_TRY(cudaMemcpy(order.data(), sc->leaf_order.ptr, size_t(n) * 4, cudaMemcpyDeviceToHost));
+    // The caller may be capturing, and its current device stays.
+    {
+        DeviceScope on(sc->device);
+        RelaxedCaptureScope relaxed;
+        cudaStream_t stream = nullptr;
+        RE_CUDA_TRY(scene_pool_stream(sc->device, &stream));
+        RE_CUDA_TRY(cudaMemcpyAsync(dev.data(), sc->nodes.ptr, dev.size() * sizeof(DeviceNode),
+                                    cudaMemcpyDeviceToHost, stream));
+        RE_CUDA_TRY(cudaMemcpyAsync(order.data(), sc->leaf_order.ptr, size_t(n) * 4, cudaMemcpyDeviceToHost, stream));
+        RE_CUDA_TRY(cudaStreamSynchronize(stream));
+    }
     std::vector<re_software_node> nodes;
     nodes.reserve(2u * size_t(n) - 1u);
     struct Item {

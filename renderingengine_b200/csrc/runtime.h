@@ -71,6 +71,29 @@ struct BuildBuffer : DeviceBuffer {
 
 // What the scene pool of `device` holds unused goes back to the device.
 void trim_scene_pool(int device);
+// The scene pool's stream, which waits for no other: for copies of a finished
+// scene's buffers beside whatever the caller's streams do.
+cudaError_t scene_pool_stream(int device, cudaStream_t* out);
+
+// Makes a device current for a scope.
+struct DeviceScope {
+    int before = 0, device;
+    explicit DeviceScope(int d) : device(d) {
+        cudaGetDevice(&before);
+        if (before != device) cudaSetDevice(device);
+    }
+    ~DeviceScope() {
+        if (before != device) cudaSetDevice(before);
+    }
+};
+
+// For a scope, this thread's calls are not held against another thread's stream
+// capture, whatever its mode.
+struct RelaxedCaptureScope {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCaptureScope() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCaptureScope() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 }  // namespace re
 

@@ -73,19 +73,14 @@ cudaError_t scene_pool(int device, ScenePool* out) {
     return cudaSuccess;
 }
 
-// Makes a device current for a scope.
-struct DeviceScope {
-    int before = 0, device;
-    explicit DeviceScope(int d) : device(d) {
-        cudaGetDevice(&before);
-        if (before != device) cudaSetDevice(device);
-    }
-    ~DeviceScope() {
-        if (before != device) cudaSetDevice(before);
-    }
-};
-
 }  // namespace
+
+cudaError_t scene_pool_stream(int device, cudaStream_t* out) {
+    ScenePool p;
+    const cudaError_t e = scene_pool(device, &p);
+    *out = p.stream;
+    return e;
+}
 
 void trim_scene_pool(int device) {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
@@ -401,12 +396,7 @@ const float4* quad_nodes(re_scene* sc, uint32_t count, cudaStream_t stream) {
         cudaGetLastError();
         return nullptr;
     }
-    // Another thread may be capturing a stream of its own.
-    struct Relaxed {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    } relaxed;
+    RelaxedCaptureScope relaxed;  // another thread may be capturing a stream of its own
     if (state == re_scene::kQuadNone) {
         std::lock_guard<std::mutex> lock(sc->quad_mutex);
         state = sc->quad_state.load(std::memory_order_relaxed);

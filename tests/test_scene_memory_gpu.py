@@ -1,5 +1,6 @@
 """Scene memory beside the caller's own work: captures of other streams, work
 in flight, and what a scene reports to hold."""
+import ctypes
 import threading
 
 import numpy as np
@@ -141,12 +142,18 @@ def test_device_batches_do_not_wait(native, any_hit, busy):
     scene.close()
 
 
+def _blocking_stream():
+    """A stream that the legacy default stream waits for, unlike torch's."""
+    import torch
+    handle = ctypes.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0
+    return torch.cuda.ExternalStream(handle.value)
+
+
 @pytest.mark.parametrize("any_hit", [False, True])
 def test_quad_nodes_made_beside_a_capture_of_a_blocking_stream(native, any_hit):
     """Beside such a capture the legacy default stream is closed.  The batch gets
     its quad nodes all the same, and the capture its end."""
-    import ctypes
-
     import torch
     scene = _scene()
     before = scene.info().device_bytes
@@ -155,11 +162,9 @@ def test_quad_nodes_made_beside_a_capture_of_a_blocking_stream(native, any_hit):
     d_rays, d_hits = _device(rays)
     x = torch.zeros(1000, device="cuda")
     torch.cuda.synchronize()
-    handle = ctypes.c_void_p()
-    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0  # blocking, unlike torch's
-    own = torch.cuda.Stream()
+    own, blocking = torch.cuda.Stream(), _blocking_stream()
     graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(handle.value), capture_error_mode="relaxed"):
+    with torch.cuda.graph(graph, stream=blocking, capture_error_mode="relaxed"):
         x.add_(1.0)
         scene.trace_device(d_rays.data_ptr(), d_hits.data_ptr(), len(rays), any_hit, stream=own.cuda_stream)
     graph.replay()
@@ -168,3 +173,34 @@ def test_quad_nodes_made_beside_a_capture_of_a_blocking_stream(native, any_hit):
     assert scene.info().device_bytes > before
     got = d_hits.cpu().numpy().view(N.HIT_DTYPE)[:1000]
     np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_export_beside_a_capture(native, mode):
+    """The first export of a tree that was built on the device."""
+    import torch
+    nodes, order = _scene().export_flat()
+    scene = _scene()
+    x = torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    graph, got = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph, stream=_blocking_stream(), capture_error_mode=mode):
+        x.add_(1.0)
+        t = threading.Thread(target=lambda: got.extend(scene.export_flat()))
+        t.start()
+        t.join()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1000.0
+    assert got[0].tobytes() == nodes.tobytes()
+    np.testing.assert_array_equal(got[1], order)
+
+
+def test_export_keeps_the_current_device(native):
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs a second GPU to be current")
+    scene = _scene()
+    with torch.cuda.device(1):
+        scene.export_flat()
+        assert torch.cuda.current_device() == 1
