@@ -679,7 +679,8 @@ __device__ __forceinline__ BsdfSample bsdf_sample_body(const BsdfContext& c, con
 // bit-identical; the parameters must have passed validate_params (the Shade
 // stage checks them before it records a vertex).
 // ---------------------------------------------------------------------------
-// EvaluateBsdfL6 of the normalised direction wi in frame f.
+// EvaluateBsdfL6 of the normalised direction wi in frame f.  (An evaluation that is
+// not valid may keep values of the steps before.)
 __device__ __forceinline__ BsdfEval evaluate_in_frame_warp(bool live, const BsdfContext& c, const BsdfParams& p,
                                                            const Frame& f, f3 wi_in) {
     BsdfEval r = bsdf_eval_invalid();
@@ -692,6 +693,7 @@ __device__ __forceinline__ BsdfEval evaluate_in_frame_warp(bool live, const Bsdf
         else if (p.model == kModelRoughDielectric) r = eval_rough_dielectric(c, p, f.wo_local, wil);
         else if (p.model == kModelGgxConductor || p.model == kModelGgxDielectricReflection)
             r = eval_ggx_reflection(c, p, f.wo_local, wil);
+        else if (p.model == kModelSmoothGlass) r.measure = kMeasureDiscrete;
     }
     __syncwarp();
     float corr = 0.f;

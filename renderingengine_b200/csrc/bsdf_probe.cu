@@ -3,6 +3,10 @@
 // query.  Counterpart of the reference's readback probe
 // resources/shaders/integrators/pbr_sampling_probe.hlsl:9-102, with the
 // context, parameters, directions and random triple chosen per query.
+//
+// The BSDF is there twice, as out-of-line calls and in the warp-wide form of the
+// default Shade kernels (bsdf.cuh).  Every other warp of queries runs the second,
+// so both stand to the same checks.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -21,8 +25,8 @@ __device__ __forceinline__ f3 xyz(float4 v) { return mk(v.x, v.y, v.z); }
 
 __global__ void __launch_bounds__(128) k_bsdf_probe(const float4* __restrict__ q, uint32_t n, float4* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4* r = q + size_t(i) * 10u;
+    const bool live = i < n, wide = (i >> 5) & 1u;
+    const float4* r = q + size_t(live ? i : n - 1u) * 10u;
     float4 v[10];
 #pragma unroll
     for (int k = 0; k < 10; ++k) v[k] = r[k];
@@ -45,13 +49,20 @@ __global__ void __launch_bounds__(128) k_bsdf_probe(const float4* __restrict__ q
     p.lobes = __float_as_uint(v[7].w);
     p.complex_fresnel = __float_as_uint(v[8].w);
     const f3 wo = xyz(v[7]), wi = xyz(v[8]), u = xyz(v[9]);
-    const BsdfEval e = bsdf_evaluate<false>(true, c, p, wo, wi);
-    const BsdfSample s = bsdf_sample<false>(true, c, p, wo, u);
-    float pdf_at = 0.f;
-    if (s.valid && !s.delta) {
-        const BsdfEval e2 = bsdf_evaluate<false>(true, c, p, wo, s.dir);
-        pdf_at = (e2.valid && e2.measure == kMeasureSolidAngle) ? e2.pdf : 0.f;
-    }
+    // The warp forms take parameters that are known to be valid.
+    const bool valid = validate_params(c, p);
+    const bool unit = finite3(u) && u.x >= 0.f && u.y >= 0.f && u.z >= 0.f && u.x < 1.f && u.y < 1.f && u.z < 1.f;
+    __syncwarp();
+    BsdfEval e = wide ? bsdf_evaluate<true>(valid, c, p, wo, wi) : bsdf_evaluate<false>(true, c, p, wo, wi);
+    if (!e.valid && e.measure != kMeasureDiscrete) e = bsdf_eval_invalid();  // as the out-of-line form leaves it
+    __syncwarp();
+    const BsdfSample s = wide ? bsdf_sample<true>(valid && unit, c, p, wo, u) : bsdf_sample<false>(true, c, p, wo, u);
+    __syncwarp();
+    const bool at_sample = s.valid && !s.delta;
+    const BsdfEval e2 = wide ? bsdf_evaluate<true>(at_sample, c, p, wo, s.dir)
+                             : bsdf_evaluate<false>(at_sample, c, p, wo, s.dir);
+    const float pdf_at = at_sample && e2.valid && e2.measure == kMeasureSolidAngle ? e2.pdf : 0.f;
+    if (!live) return;
     float4* o = out + size_t(i) * 8u;
     o[0] = make_float4(e.value.x, e.value.y, e.value.z, e.pdf);
     o[1] = make_float4(e.diffuse.x, e.diffuse.y, e.diffuse.z, __uint_as_float(e.measure));
