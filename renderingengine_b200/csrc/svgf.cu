@@ -435,8 +435,10 @@ __global__ void __launch_bounds__(256) k_temporal(TemporalArgs a) {
     a.pl.reject[i] = reject;
 
     // Edge record shared by the bootstrap and every A-Trous iteration.
-    const bool filterable = gb_valid(g) && geom;
+    // (A normal whose length overflows normalises to zero, which has no weight
+    // with any other; edge_exponent wants unit normals.)
     const V3 nn = normalize_safe(g.n);
+    const bool filterable = gb_valid(g) && geom && dot(nn, nn) > 0.5F;
     a.pl.edge[i] = make_float4(nn.x, nn.y, nn.z, filterable ? g.depth : -1.0F);
     a.pl.ids[i] = make_uint2(g.mat, g.obj);
     // First inputs of the two chains: the temporal signal (SVGF) and the
