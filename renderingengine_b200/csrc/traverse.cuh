@@ -1513,7 +1513,7 @@ __device__ __forceinline__ TraceHit trace_coop(const TraceSceneView& s, const Tr
     if (lane == 0u) stack[0] = make_uint2(0u, 0u);
     __syncwarp();
     uint32_t steps = 0u;
-    const uint32_t max_steps = s.wide_count * 5u + 8u;
+    const uint32_t max_steps = s.wide_count * 6u + 8u;  // nodes, their leaves and marks
     while (sp > 0) {
         if (++steps > max_steps) {  // malformed (cyclic) tree guard
             h.status = 3u;
