@@ -87,13 +87,14 @@ class ClockSampler:
 
 # DRAM bytes (read + write) of the 8 k_intersect launches of one frame of the
 # frame workload, by hierarchy and node layout, from one ncu capture each of
-# this command with --tuning b200_frame_lbvh (dram__bytes_read.sum +
-# dram__bytes_write.sum, mean of two frames that agree within 0.6 %), with the
+# two frames of perf/cases.py's frame_heightfield_1080p, the same frame with the
+# same tuning (build "sah" for the second) (dram__bytes_read.sum +
+# dram__bytes_write.sum, mean of two frames that agree within 0.7 %), with the
 # source revision the capture ran.  Not measured by the run itself: ncu is not
 # available inside it.  Layouts without a capture report null.
 INTERSECT_DRAM_BYTES_PER_FRAME = {
-    ("lbvh", "four-wide"): (573.9e6, "ncu capture, source of commit ad76b66, k_intersect<64, 4, 512>"),
-    ("sah", "four-wide"): (498.3e6, "ncu capture, source of commit ad76b66, k_intersect<64, 2, 512>"),
+    ("lbvh", "four-wide"): (563.9e6, "ncu capture, source of commit 55ce86b, k_intersect<64, 4, 512>"),
+    ("sah", "four-wide"): (491.5e6, "ncu capture, source of commit 55ce86b, k_intersect<64, 2, 512>"),
 }
 NODE_LAYOUT = {0: "child-pair", 1: "child-pair", 2: "four-wide", 4: "four-wide", 5: "eight-wide",
                6: "eight-wide-compressed", 7: "four-wide-conservative", 8: "four-wide-conservative"}
@@ -1045,7 +1046,7 @@ def main() -> None:
         # One trace launch per step: its event time is the step's.
         alg = wl.algorithmic_bytes()
         achieved = alg / (ms_max / args.steps / 1e3) / 1e9
-        kernel = "trace_batch_kernel (one launch per step)"
+        kernel = "trace_quad_kernel (one launch per step)"
     l2_view = ({"peak": round(l2_gbs, 1), "unit": "GB/s", "frac": round(achieved / l2_gbs, 4),
                 "how": "device copy of a 24 MiB L2-resident buffer, read + write bytes, best of 3 x 100, CUDA events"}
                if l2_gbs else {"unavailable": l2_err})

@@ -205,10 +205,12 @@ __device__ __forceinline__ RisFold ris_fold(const WfDevice& d, const FrameParams
         // whether it is valid and its weight: the light sample is inlined so
         // its unused fields and the numbers its type does not take (two of
         // five draws for a triangle or a sphere) are never computed, and the
-        // surface's share of the target is computed once.  Bound by
-        // instruction issue.  1280x720: 1,380 us
-        // a frame with every number drawn and the surface's share computed per
-        // candidate, 880 us without them (667 with the launch's pixels balanced).
+        // surface's share of the target is computed once.  Issues in half of
+        // the cycles for 15 of 32 lanes (a warp's light types take turns) and
+        // waits for light records and alias entries read at random.  1280x720:
+        // 1,380 us a frame with every number drawn and the surface's share
+        // computed per candidate, 880 us without them (667 with the launch's
+        // pixels balanced).
         const RisSurface rsurf = ris_surface(s, fp.cam_pos);
 #pragma unroll 1
         for (uint32_t c = 0; c < C; ++c) {

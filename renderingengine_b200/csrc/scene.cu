@@ -319,10 +319,12 @@ __global__ void __launch_bounds__(128) trace_batch_kernel(BatchArgs args) {
 }
 
 // Batch over the quad nodes: trace_batch_kernel<ANY, false>'s hits, in its order
-// of visits, from half the dependent node fetches.  2,073,600 closest-hit rays
-// over 2,424,832 triangles: camera rays 895 us over the child pairs, 814 here,
-// random rays 1,265 and 1,104; 400,009 random any-hit rays over 60,000
-// triangles: 668 and 529.
+// of visits, from half the dependent node fetches.  Bound by instruction issue for
+// few lanes: 66 % of the cycles for 6 of 32 lanes on random any-hit rays, 72 % for
+// 14 on camera rays; the rest waits for nodes.  2,073,600 closest-hit rays over
+// 2,424,832 triangles: camera rays 895 us over the child pairs, 814 here, random
+// rays 1,265 and 1,104; 400,009 random any-hit rays over 60,000 triangles: 668 and
+// 529.
 template <bool ANY, int STACK>
 __global__ void __launch_bounds__(128, 8) trace_quad_kernel(BatchArgs args) {
     for (WarpWork w(args.count); w.more(); w.next(args.work)) {

@@ -505,7 +505,7 @@ constexpr float kLog2E = 1.44269504F;
 // length 1 and variance 0.  The bootstrapped variances go into the chains'
 // first inputs, where the first A-Trous iteration reads them.
 //
-// Bound by instruction issue over 49 taps a pixel: a tap reads 32 bytes (edge,
+// Bound by instruction issue (82 % of the cycles) over 49 taps a pixel: a tap reads 32 bytes (edge,
 // IDs, both luminances; NaN marks a luminance that must not count) in place of
 // 88 and takes one exponential in place of expf and powf.  1280x720, radius 3:
 // 272 us with the exponentials taken one by one, 104 us now.
@@ -598,10 +598,11 @@ __host__ __device__ __forceinline__ uint32_t atrous_row_stride(uint32_t step, ui
 // only a luminance may overflow, and then the weight is 0 or NaN, and NaN is
 // made 0.  LAST remodulates into the frame's atrous / svgf planes.
 //
-// Bound by instruction issue and L1 (25 taps of 88 bytes).  1280x720, five
-// iterations of a frame: 1,666 us before the packed form, 631 us now.  Held to
-// 64 registers (four CTAs per SM) a whole reconstruction takes 1,586 us, with
-// the registers that the compiler picks by itself 1,707.
+// Bound by the latency of its taps' loads (25 of 88 bytes): four CTAs per SM issue
+// in 54 % of the cycles at step 1 and 40 % at step 16, where 71 % of the loads hit
+// the L1.  1280x720, five iterations of a frame: 1,666 us before the packed form,
+// 631 us now.  Held to 64 registers (four CTAs per SM) a whole reconstruction takes
+// 1,586 us, with the registers that the compiler picks by itself 1,707.
 template <bool LAST>
 __global__ void __launch_bounds__(kAtrousX * kAtrousY, 4) k_atrous(FilterArgs a, int step, int ping) {
     const int W = int(a.W), H = int(a.H);

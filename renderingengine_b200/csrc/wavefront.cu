@@ -1181,7 +1181,8 @@ __global__ void __launch_bounds__(128, shade_min_blocks(VARIANT)) k_shade(WfDevi
 // (material parameters, shading frame, view direction) and samples the
 // BSDF, so the next ray is the one the one-kernel Shade emits.
 //
-// Bound by instruction issue and fetch.  All lanes of a warp go through the BSDF
+// Bound by latency: 10 to 15 warps per SM issue in 20 to 38 % of the cycles and
+// wait for records and for instructions.  All lanes of a warp go through the BSDF
 // together (bsdf_*_warp: branches take turns, then the lanes meet again), and
 // each kernel is held to 128 registers, four CTAs per SM: k_shade_b of a 1080p
 // heightfield frame takes 302 / 153 / 115 us at bounces 0 / 1 / 2 in place of
