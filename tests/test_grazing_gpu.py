@@ -94,3 +94,30 @@ def test_grazing_warp_per_ray_equals_lane_per_ray(native, build, seed, side, clu
         planes.append(_planes(scene, data, _views(data, o, forward), len(o), mode))
     for a, b in zip(*planes):
         assert not (a != b).any(), f"{(a != b).any(1).sum()} of {len(o)} views"
+
+
+@pytest.mark.parametrize("mode", [2, 4])
+@pytest.mark.parametrize("shrink", [0.5, 0.8, 1.0])
+def test_callers_leaf_boxes_smaller_than_their_triangles(native, shrink, mode):
+    """A caller's tree whose leaf boxes lie within their parents' but do not hold
+    their triangles: hits far before their boxes, warp against lane as above."""
+    data = scenes.heightfield_scene(grid=48, spheres=48, seed=2)
+    far = scenes.canonical_triangles(np.array([[[50, 0, 0], [50, 1, 0], [50, 0, 1]]], np.float32), None, np.zeros(1, np.uint32),
+                                     np.full(1, 1 << 20, np.uint32), data.triangles["identity"][:1, 3],
+                                     first_traversal_id=len(data.triangles))
+    data.triangles = np.concatenate([data.triangles, far])
+    nodes, order = Scene(data.triangles, data.fingerprint).export_flat()
+    leaf = nodes["links"][:, 1] > 0
+    centre = (nodes["bounds_min"][leaf] + nodes["bounds_max"][leaf]) / 2
+    for b in ("bounds_min", "bounds_max"):
+        nodes[b][leaf] = centre + (nodes[b][leaf] - centre) * np.float32(shrink)
+    data.triangles = np.ascontiguousarray(data.triangles[order])
+    at = int(np.argmax(data.triangles["positions"][:, 0, 0]))
+    view = dict(frame=frame_constants(data.camera, 118, 80, 0, 4, seed=0x51), offset=0, key=0)
+    planes = []
+    for masked in (False, True):
+        data.triangles["metadata"][at, 0] |= 2 * masked  # RE_GEOMETRY_FLAG_ALPHA_MASK
+        scene = Scene(data.triangles, data.fingerprint, 1, N.BUILD_FLATTENED_SAH, nodes=nodes)
+        planes.append(_planes(scene, data, [view], 118 * 80, mode))
+    for a, b in zip(*planes):
+        assert not (a != b).any(), f"{(a != b).any(1).sum()} of {118 * 80} pixels"
